@@ -293,23 +293,23 @@ __global__ void summarize_kernel(uint64_t *__restrict__ h1, uint64_t *__restrict
 			while (x) {
 				uint32_t f = w * 64 + (uint32_t)(__ffsll((long long)x) - 1);
 				x &= x - 1;
-				atomicAdd(&sc[f], 1ull);
+				atomicAdd(&sc[f], 1u);
 				idx = idx == nf ? f : nf + 1;
 			}
 		}
 		if (idx == nf)
-			atomicAdd(&sc[2 * (nf + 2) + 1], 1ull);
+			atomicAdd(&sc[2 * (nf + 2) + 1], 1u);
 		else if (idx == nf + 1)
-			atomicAdd(&sc[2 * (nf + 2)], 1ull);
+			atomicAdd(&sc[2 * (nf + 2)], 1u);
 		else
-			atomicAdd(&sc[(nf + 2) + idx], 1ull);
+			atomicAdd(&sc[(nf + 2) + idx], 1u);
 		if (category)
 			category[i] = idx;
 	}
 	__syncthreads();
 	for (uint32_t j = threadIdx.x; j < ncount; j += blockDim.x)
 		if (sc[j])
-			atomicAdd(&counts[j], sc[j]);
+			atomicAdd(&counts[j], (unsigned long long)sc[j]);
 }
 
 /* Warp-aggregated split of the reads into long (front of order, in counter 0)
@@ -475,7 +475,7 @@ cudaError_t launch_summarize(uint64_t *h1, uint64_t *h2, uint64_t n, uint32_t nf
 	uint64_t need = (n + threads - 1) / threads;
 	uint64_t cap = (uint64_t)num_sms * 4;
 	unsigned blocks = (unsigned)(need < cap ? need : cap);
-	size_t smem = sizeof(unsigned long long) * (2 * (nf + 2) + 2);
+	size_t smem = sizeof(uint32_t) * (2 * (nf + 2) + 2);
 	summarize_kernel<<<blocks, threads, smem, s>>>(h1, h2, n, nf, words, inclusive, ordered,
 			category, counts);
 	return cudaGetLastError();
