@@ -25,7 +25,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 DEFINES = os.environ.get("BBT_BUILD_DEFINES", "").split()
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC,
           "-Xcompiler", "-fPIC,-fopenmp,-O3,-Wall", "-ccbin", "/usr/bin/g++"] + DEFINES
-LIB_SOURCES = ["classify.cu", "score.cu", "dust.cu", "twopass.cu", "bucketed.cu", "api.cu", "noalloc.cu", "gather_rate.cu", "maker.cu", "mibf.cu",
+LIB_SOURCES = ["classify.cu", "lane.cu", "score.cu", "dust.cu", "twopass.cu", "bucketed.cu", "api.cu", "noalloc.cu", "gather_rate.cu", "maker.cu", "mibf.cu",
                "mibf_make.cu", "formats.cpp", "pack.cpp", "fastx.cpp", "synth.cpp", "mibf_host.cpp",
                "mibf_pipeline.cpp", "server.cpp"]
 CLIS = [("biobloomcategorizer", "cli_categorizer.cpp"),

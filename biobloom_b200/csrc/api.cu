@@ -22,6 +22,7 @@
 #include "classify.cuh"
 #include "ctx.hpp"
 #include "formats.hpp"
+#include "lane.cuh"
 #include "twopass.cuh"
 
 namespace bbt {
@@ -178,6 +179,7 @@ extern "C" int bbt_close(bbt_ctx *ctx)
 	cudaFree(ctx->d_work);
 	cudaFree(ctx->d_order);
 	cudaFree(ctx->d_order_cnt);
+	cudaFree(ctx->d_lane_list);
 	cudaFree(ctx->d_bthres);
 	cudaFree(ctx->d_lenset);
 	cudaFree(ctx->d_stat);
@@ -520,7 +522,8 @@ extern "C" int bbt_open(const char *const *bf_paths, int n_filters, const bbt_pa
 	OPEN_TRY(cudaMalloc(&ctx->d_counts, sizeof(unsigned long long) * (2 * (ctx->nf + 2) + 2)));
 	OPEN_TRY(cudaMemset(ctx->d_counts, 0, sizeof(unsigned long long) * (2 * (ctx->nf + 2) + 2)));
 	OPEN_TRY(cudaMalloc(&ctx->d_work, sizeof(unsigned long long)));
-	OPEN_TRY(cudaMalloc(&ctx->d_order_cnt, 2 * sizeof(unsigned long long)));
+	OPEN_TRY(cudaMalloc(&ctx->d_order_cnt, order_counters(ctx->nf) *
+			sizeof(unsigned long long)));
 	OPEN_TRY(cudaMalloc(&ctx->d_stat, 3 * sizeof(unsigned long long)));
 	OPEN_TRY(cudaMemset(ctx->d_stat, 0, 3 * sizeof(unsigned long long)));
 	ctx->cap_reads = ctx->p.max_batch_reads ? ctx->p.max_batch_reads : (1ull << 20);
@@ -1196,6 +1199,36 @@ static int dust_check(bbt_ctx *ctx)
 	return BBT_OK;
 }
 
+/* Whether these launches take the lane kernel: the persistent path with its
+ * default steps and the filter-major path, filters and options that it
+ * supports, and enough reads. */
+static bool lane_wanted(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t total)
+{
+	const bool path = lc.path == BBT_PATH_FILTER_MAJOR ||
+			(lc.path == BBT_PATH_PERSISTENT && lc.steps == BBT_STEPS_DECISION);
+	return path && lane_pays(total) &&
+			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total);
+}
+
+/* The lane kernel over a batch: hits (classify) and / or scores (sa). */
+static int run_lane(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreArgs *sa,
+		bool classify)
+{
+	const LaneScratch ls = {ctx->d_lane_list, ctx->d_order_cnt};
+	if (classify) {
+		const size_t hb = a.n * ctx->words * sizeof(uint64_t);
+		for (uint32_t m = 0; ctx->nf > 1 && m < a.mates; ++m)
+			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
+		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, ls, ctx->num_sms, ctx->lc.count != 0, s));
+		ctx->last.kernels += 1 + ctx->nf;
+	}
+	if (sa) {
+		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), sa, ls, ctx->num_sms, false, s));
+		ctx->last.kernels += 1 + ctx->nf;
+	}
+	return BBT_OK;
+}
+
 /* classify + summarize one staged or device-resident batch on stream s;
  * scores (optional, per mate array): evalScore of every filter */
 static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStream_t s,
@@ -1216,12 +1249,30 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	sa.besthit = 0;
 	bool want_scores = sa.scores[0] || sa.scores[1];
 	const bool two_pass = ctx->lc.path == BBT_PATH_FILTER_MAJOR && ctx->same_k;
+	const bool best_only = ctx->mode == BBT_MODE_BESTHIT && !want_scores;
+	bool lane = lane_wanted(ctx, ctx->lc, a.n * a.mates);
+	/* BESTHIT through stored scores: outside the filter-major path, whose
+	 * batches always stored them, only while they stay within 1 GB */
+	if (lane && best_only && !two_pass && a.n * ctx->nf * a.mates > (128ull << 20))
+		lane = false;
+	/* scores of one mate only: the kernels that test each array */
+	if (lane && want_scores && (!sa.scores[0] || (a.mates == 2 && !sa.scores[1])))
+		lane = false;
+	/* no allocation while a graph is captured */
+	if (lane && ctx->capturing && (a.n * a.mates > ctx->lane_list_cap ||
+			(best_only && a.n * ctx->nf > ctx->tmp_scores_cap)))
+		lane = false;
+	if (lane) {
+		int rc = grow(ctx, &ctx->d_lane_list, ctx->lane_list_cap, a.n * a.mates);
+		if (rc)
+			return rc;
+	}
 	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_k0, s));
-	if (two_pass && (ctx->mode == BBT_MODE_BESTHIT || want_scores)) {
+	if ((lane || two_pass) && (ctx->mode == BBT_MODE_BESTHIT || want_scores)) {
 		/* filter-major score pass (and filter pass for the hits unless
 		 * BESTHIT, whose hits come from the scores) */
 		ScoreArgs ps = sa;
-		if (ctx->mode == BBT_MODE_BESTHIT && !want_scores) {
+		if (best_only) {
 			const uint64_t need = a.n * ctx->nf;
 			if (need > ctx->tmp_scores_cap) {
 				cudaFree(ctx->d_tmp_scores[0]);
@@ -1236,14 +1287,14 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 			ps.scores[1] = a.mates == 2 ? ctx->d_tmp_scores[1] : nullptr;
 		}
 		const bool classify = ctx->mode != BBT_MODE_BESTHIT;
-		if (classify) {
+		if (classify && !lane) {
 			const size_t hb = a.n * ctx->words * sizeof(uint64_t);
 			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[0], 0, hb, s));
 			if (a.mates == 2)
 				CUDA_TRY(ctx, cudaMemsetAsync(a.hits[1], 0, hb, s));
 		}
 		ctx->last.kernels -= 1; /* the passes count themselves */
-		int rc = run_two_pass(ctx, a, s, &ps, classify);
+		int rc = lane ? run_lane(ctx, a, s, &ps, classify) : run_two_pass(ctx, a, s, &ps, classify);
 		if (rc)
 			return rc;
 		if (!classify) {
@@ -1258,6 +1309,11 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	} else if (ctx->lc.path == BBT_PATH_BUCKETED && !want_scores) {
 		ctx->last.kernels -= 1; /* the passes count themselves */
 		int rc = run_bucketed(ctx, a, s);
+		if (rc)
+			return rc;
+	} else if (lane) {
+		ctx->last.kernels -= 1;
+		int rc = run_lane(ctx, a, s, nullptr, true);
 		if (rc)
 			return rc;
 	} else if (two_pass) {
@@ -2209,6 +2265,11 @@ extern "C" int bbt_graph_create(bbt_ctx *ctx, const bbt_batch *b, const bbt_resu
 		if (rc)
 			return rc;
 	}
+	if (lane_wanted(ctx, ctx->lc, chunk * (b->seq2 ? 2 : 1))) {
+		int rc = grow(ctx, &ctx->d_lane_list, ctx->lane_list_cap, chunk * (b->seq2 ? 2 : 1));
+		if (rc)
+			return rc;
+	}
 	if (ctx->p.scoring == BBT_SCORE_BINOMIAL) { /* thresholds before capture */
 		std::vector<uint64_t> lens;
 		int rc = device_lengths(ctx, b, ctx->stream, lens);
@@ -2297,7 +2358,8 @@ int bbt::bf_scratch_init(bbt_ctx *ctx, BfScratch &sc, uint64_t max_reads)
 {
 	CUDA_TRY(ctx, cudaSetDevice(ctx->dev));
 	CUDA_TRY(ctx, cudaMalloc(&sc.work, sizeof(unsigned long long)));
-	CUDA_TRY(ctx, cudaMalloc(&sc.order_cnt, 2 * sizeof(unsigned long long)));
+	CUDA_TRY(ctx, cudaMalloc(&sc.order_cnt, order_counters(ctx->nf) *
+			sizeof(unsigned long long)));
 	CUDA_TRY(ctx, cudaMalloc(&sc.order, std::max<uint64_t>(max_reads, 1) * 2 * sizeof(uint64_t)));
 	sc.order_cap = std::max<uint64_t>(max_reads, 1) * 2;
 	return BBT_OK;
@@ -2335,7 +2397,15 @@ int bbt::bf_classify_slot(bbt_ctx *ctx, const uint8_t *seq, const uint64_t *off,
 	lc.count = 0;
 	if (lc.path == BBT_PATH_FILTER_MAJOR)
 		lc.path = BBT_PATH_PERSISTENT;
-	if (ctx->mode == BBT_MODE_BESTHIT) {
+	const bool lane = ctx->mode != BBT_MODE_BESTHIT && n * a.mates <= sc.order_cap &&
+			lane_wanted(ctx, lc, n * a.mates);
+	if (lane) {
+		const size_t hb = n * ctx->words * sizeof(uint64_t);
+		for (uint32_t m = 0; ctx->nf > 1 && m < a.mates; ++m)
+			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
+		const LaneScratch ls = {reinterpret_cast<uint32_t *>(sc.order), sc.order_cnt};
+		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, ls, ctx->num_sms, false, s));
+	} else if (ctx->mode == BBT_MODE_BESTHIT) {
 		ScoreArgs sa;
 		sa.scores[0] = sa.scores[1] = nullptr;
 		sa.fpr = ctx->d_fpr;
@@ -2350,7 +2420,7 @@ int bbt::bf_classify_slot(bbt_ctx *ctx, const uint8_t *seq, const uint64_t *off,
 			a.order = sc.order;
 		}
 	}
-	if (ctx->mode != BBT_MODE_BESTHIT)
+	if (ctx->mode != BBT_MODE_BESTHIT && !lane)
 		CUDA_TRY(ctx, launch_classify(a, lc, s));
 	CUDA_TRY(ctx, launch_summarize(a.hits[0], paired ? a.hits[1] : nullptr, n, ctx->nf,
 			ctx->words, ctx->p.inclusive, ctx->mode == BBT_MODE_ORDERED, category,

@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -13,6 +14,7 @@
 #include "bbt.h"
 #include "classify.cuh"
 #include "dust.cuh"
+#include "lane.cuh"
 
 namespace bbt {
 
@@ -112,7 +114,10 @@ struct bbt_ctx {
 	uint64_t long_bases = 0;
 	uint64_t *d_order = nullptr;
 	uint64_t order_cap = 0;
-	unsigned long long *d_order_cnt = nullptr;
+	unsigned long long *d_order_cnt = nullptr; /* order_counters(nf) words */
+	/* lane kernel (lane.cu): the batch's long reads */
+	uint32_t *d_lane_list = nullptr;
+	uint64_t lane_list_cap = 0;
 	/* bucketed probe path (bucketed.cu): frame offsets of a batch's reads and
 	 * their host samples, per-read state, the batch's bases as 2-bit codes
 	 * (ASCII batches), validity / hit / requesting bits and canonical hashes
@@ -155,6 +160,11 @@ struct bbt_ctx {
 };
 
 namespace bbt {
+/* Counters of the read order (2) or of the lane kernel. */
+inline size_t order_counters(uint32_t nf)
+{
+	return std::max<size_t>(2, lane_counters(nf));
+}
 int fail(bbt_ctx *ctx, int code, const std::string &msg);
 
 /* Per-stream scratch for classification calls that run concurrently on
