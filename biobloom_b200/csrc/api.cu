@@ -733,6 +733,8 @@ static ClassifyArgs base_args(const bbt_ctx *ctx)
 	a.bthres = ctx->d_bthres;
 	a.bthres_rows = ctx->bt_rows;
 	a.work = ctx->d_work;
+	a.lane_long = ctx->lc.steps == BBT_STEPS_DECISION &&
+			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, 0);
 	if (ctx->lc.count) {
 		a.probes = ctx->d_stat;
 		a.frames = ctx->d_stat + 1;
@@ -1200,13 +1202,13 @@ static int dust_check(bbt_ctx *ctx)
 }
 
 /* Whether these launches take the lane kernel: the persistent path with its
- * default steps and the filter-major path, filters and options that it
- * supports, and enough reads. */
+ * default steps and the filter-major path, with filters and options that it
+ * supports, for enough reads. */
 static bool lane_wanted(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t total)
 {
 	const bool path = lc.path == BBT_PATH_FILTER_MAJOR ||
 			(lc.path == BBT_PATH_PERSISTENT && lc.steps == BBT_STEPS_DECISION);
-	return path && lane_pays(total) &&
+	return path && lane_pays(ctx->hf.data(), ctx->nf, total) &&
 			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total);
 }
 

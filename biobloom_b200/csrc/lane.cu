@@ -18,7 +18,7 @@
  * one filter at a time and a filter that fits L2 stays there; warps take chunks
  * of 32 reads from a counter.  A warp keeps its next items (base position,
  * length, thresholds: computed 32 at a time) in shared memory and hands them to
- * lanes as these finish.  Reads above kLaneMaxBases would leave a lane working
+ * lanes as these finish.  Reads above LaneArgs::max_bases would leave a lane working
  * long after its warp and are evaluated by whole warps, before the others: a
  * small kernel lists them.
  */
@@ -27,16 +27,12 @@
 #include <algorithm>
 
 #include "bbt.h"
-#include "classify_read.cuh"
-#include "lane_walk.cuh"
-#include "score_value.cuh"
+#include "lane_item.cuh"
 
 namespace bbt {
 
 namespace {
 
-constexpr uint64_t kLaneMaxBases = 1024;
-constexpr uint64_t kLaneKeepBytes = 126ull << 20; /* L2 */
 constexpr int kLaneWarps = 8;     /* warps per block */
 /* Blocks per SM the registers leave room for: 3 give a thread 80, which hold
  * eight frames' hashes and words in flight without spills (4 blocks spill, and
@@ -59,10 +55,8 @@ struct LaneArgs {
 	unsigned long long *ctr;    /* next chunk, next long read */
 	uint64_t chunks;
 	uint32_t f;                 /* the filter's index */
-	uint32_t k, h, m5, inv_hi, inv_lo;
-	uint64_t kmul;
-	const uint32_t *words;
-	uint32_t keep;              /* the filter fits L2 */
+	LaneFilter F;
+	uint32_t max_bases;         /* of a lane's read */
 };
 
 /* What a lane needs of its read once per eight bases or less, and the bases
@@ -79,23 +73,9 @@ struct LaneWarp {
 	double hthres[MODE == SCORE_HARMONIC ? 32 : 1], my_hthres[MODE == SCORE_HARMONIC ? 32 : 1];
 };
 
-template <int MODE>
-__host__ __device__ inline size_t lane_warp_bytes(uint32_t kmax)
-{
-	const size_t win = window_stride<4>(kmax);
-	const size_t own = (sizeof(LaneWarp<MODE>) + 15) & ~(size_t)15;
-	return win > own ? win : own;
-}
-
-/* Rolling tables of the filter's k, by outgoing code << 2 | incoming code, and
- * the hashes of k bases of code 0. */
-struct LaneTables {
-	uint64_t fw[16], rc[16];
-	uint64_t f0, r0;
-};
-
-/* Indexes of the reads above kLaneMaxBases. */
-__global__ void lane_long_kernel(ClassifyArgs a, uint32_t *list, unsigned long long *nlong)
+/* Indexes of the reads above max_bases. */
+__global__ void lane_long_kernel(ClassifyArgs a, uint32_t max_bases, uint32_t *list,
+		unsigned long long *nlong)
 {
 	const uint64_t total = a.n * a.mates;
 	const int lane = threadIdx.x & 31;
@@ -106,7 +86,7 @@ __global__ void lane_long_kernel(ClassifyArgs a, uint32_t *list, unsigned long l
 		if (r < total) {
 			const uint32_t mate = r >= a.n ? 1u : 0u;
 			const uint64_t i = r - (mate ? a.n : 0);
-			is_long = a.off[mate][i + 1] - a.off[mate][i] > kLaneMaxBases;
+			is_long = a.off[mate][i + 1] - a.off[mate][i] > max_bases;
 		}
 		const unsigned m = __ballot_sync(kFull, is_long);
 		if (m) {
@@ -118,176 +98,6 @@ __global__ void lane_long_kernel(ClassifyArgs a, uint32_t *list, unsigned long l
 				list[b + __popc(m & ((1u << lane) - 1u))] = (uint32_t)r;
 		}
 	}
-}
-
-/* Seeds by base code: ASCII codes are (byte >> 1) & 3 (A, C, T, G), packed
- * ones A, C, G, T. */
-template <bool PACKED>
-__device__ __forceinline__ uint64_t lane_seed(int c, bool complement)
-{
-	const int x = PACKED ? c : c ^ (c >> 1); /* to A, C, G, T */
-	return complement ? seed_rc_of_code(x) : seed_fw_of_code(x);
-}
-
-/* The tables, by the first warp of a block. */
-template <bool PACKED>
-__device__ void lane_tables(LaneTables &t, unsigned k, int lane)
-{
-	if (lane < 16) {
-		const int out = lane >> 2, in = lane & 3;
-		t.fw[lane] = rolk(lane_seed<PACKED>(out, false), k) ^ lane_seed<PACKED>(in, false);
-		t.rc[lane] = ror1(lane_seed<PACKED>(out, true)) ^
-				rolk(lane_seed<PACKED>(in, true), k - 1);
-	}
-	uint64_t f = lane < (int)k ? rolk(lane_seed<PACKED>(0, false), lane) : 0ull;
-	uint64_t r = lane < (int)k ? rolk(lane_seed<PACKED>(0, true), lane) : 0ull;
-	for (int o = 16; o; o >>= 1) {
-		f ^= __shfl_xor_sync(kFull, f, o);
-		r ^= __shfl_xor_sync(kFull, r, o);
-	}
-	if (lane == 0) {
-		t.f0 = f;
-		t.r0 = r;
-	}
-}
-
-/* A filter word, not kept in L1 (an SM seldom probes a line twice, and the lines
- * would push out the reads' bases), with the L2 policy of lane_policy. */
-__device__ __forceinline__ uint32_t lane_probe(const uint32_t *p, uint64_t pol)
-{
-	uint32_t v;
-	asm("ld.global.nc.L1::no_allocate.L2::cache_hint.b32 %0, [%1], %2;"
-			: "=r"(v) : "l"(p), "l"(pol));
-	return v;
-}
-
-/* L2 policy of a filter's words: kept against everything else when the filter
- * fits L2 (no_allocate alone also makes L2 drop the line early: the ten filters
- * of 68 MB then took 17.7 ms per 400k pairs instead of 8.7), the first to go
- * when it does not (the reads' bases stay: 9.7 -> 9.3 ms per 2M reads over a
- * 2.1 GB filter). */
-__device__ __forceinline__ uint64_t lane_policy(bool keep)
-{
-	uint64_t last, first;
-	asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(last));
-	asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(first));
-	return keep ? last : first;
-}
-
-__device__ __forceinline__ uint32_t lane_ld(const uint32_t *p, uint64_t pol)
-{
-	uint32_t v;
-	asm("ld.global.nc.L2::cache_hint.b32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
-	return v;
-}
-
-/* Eight bases of a read from base g of its mate array, nb of them before its
- * end: nibbles (code of base j at bits 4j) and a mask of bases that are not
- * ACGT.  Loads are aligned 4-byte words, none of which lies wholly past the
- * read; the lines are in L1 from one call to the next. */
-template <bool PACKED>
-__device__ __forceinline__ void lane_bases(const ClassifyArgs &a, uint32_t mate, uint64_t g,
-		uint32_t nb, uint32_t &nib, uint32_t &bad)
-{
-	const uint64_t pol = evict_first_policy(); /* the next filter reads them again, much later */
-	if (PACKED) {
-		const uint32_t *p = reinterpret_cast<const uint32_t *>(a.seq[mate]) + (g >> 4);
-		const uint32_t at = (uint32_t)(g & 15u);
-		const uint32_t c0 = lane_ld(p, pol), c1 = at + nb > 16u ? lane_ld(p + 1, pol) : 0u;
-		uint32_t x = __funnelshift_r(c0, c1, 2u * at) & 0xFFFFu;
-		x = (x | (x << 8)) & 0x00FF00FFu;
-		x = (x | (x << 4)) & 0x0F0F0F0Fu;
-		nib = (x | (x << 2)) & 0x33333333u;
-		bad = 0;
-		if (a.valid[mate]) {
-			const uint32_t *v = a.valid[mate] + (g >> 5);
-			const uint32_t vat = (uint32_t)(g & 31u);
-			const uint32_t v0 = lane_ld(v, pol), v1 = vat + nb > 32u ? lane_ld(v + 1, pol) : 0u;
-			bad = ~__funnelshift_r(v0, v1, vat) & 0xFFu;
-		}
-		return;
-	}
-	const uintptr_t q = (uintptr_t)(a.seq[mate] + g);
-	const uint32_t *p = (const uint32_t *)(q & ~(uintptr_t)3);
-	const uint32_t at = (uint32_t)(q & 3u), end = at + nb;
-	const uint32_t w0 = lane_ld(p, pol), w1 = end > 4u ? lane_ld(p + 1, pol) : 0u;
-	const uint32_t w2 = end > 8u ? lane_ld(p + 2, pol) : 0u;
-	const uint32_t x = __funnelshift_r(w0, w1, 8u * at), y = __funnelshift_r(w1, w2, 8u * at);
-	const uint32_t cx = (x >> 1) & 0x03030303u, cy = (y >> 1) & 0x03030303u;
-	nib = __byte_perm(cx | (cx >> 4), cy | (cy >> 4), 0x6420);
-	/* the bytes those codes stand for ("ACTG"), against the bytes read */
-	const uint32_t dx = (x & 0xDFDFDFDFu) ^ __byte_perm(0x47544341u, 0, nib & 0xFFFFu);
-	const uint32_t dy = (y & 0xDFDFDFDFu) ^ __byte_perm(0x47544341u, 0, nib >> 16);
-	bad = 0;
-	if (dx | dy) {
-#pragma unroll
-		for (int j = 0; j < 4; ++j) {
-			bad |= ((dx >> (8 * j)) & 0xFFu) ? 1u << j : 0u;
-			bad |= ((dy >> (8 * j)) & 0xFFu) ? 16u << j : 0u;
-		}
-	}
-}
-
-/* One long read by the whole warp: its decision, or its score. */
-template <int MODE, bool SCORE, bool COUNT>
-__device__ __noinline__ void lane_long_item(const LaneArgs &g, uint64_t r, unsigned char *wmem,
-		int lane, unsigned long long *acc)
-{
-	const ClassifyArgs &a = g.a;
-	const uint32_t f = g.f;
-	const Window<4> win = window_at<4>(wmem);
-	const uint32_t mate = r >= a.n ? 1u : 0u;
-	const uint64_t i = r - (mate ? a.n : 0);
-	if (!SCORE) {
-		uint64_t word = 0;
-		unsigned long long words = 0, frames = 0, alg = 0;
-		classify_read<4, COUNT, MODE, true>(a, r, f, f + 1, win, lane, word, words, frames, alg);
-		if (COUNT) {
-			acc[0] += words;
-			acc[1] += frames;
-			acc[2] += alg;
-		}
-		if (lane == (int)(f >> 6)) {
-			unsigned long long *h = (unsigned long long *)&a.hits[mate][i * a.words + lane];
-			if (a.nf == 1)
-				*h = word;
-			else if (word)
-				atomicOr(h, word);
-		}
-		return;
-	}
-	const FilterDev F = a.filters[f];
-	const uint64_t start = a.off[mate][i] - a.off_base[mate];
-	const uint64_t len = a.off[mate][i + 1] - a.off[mate][i];
-	const Bases s = read_bases(a, mate, start);
-	ScoreState st;
-	score_init(st);
-	unsigned reads = 0;
-	if (len >= F.k) {
-		const uint64_t frames = len - F.k + 1;
-		set_tables<4>(win, F.k, lane);
-		for (uint64_t w0 = 0; w0 < frames; w0 += Window<4>::W) {
-			const int wn = (int)min((uint64_t)Window<4>::W, frames - w0);
-			hash_window<4>(s, w0, wn, F.k, win, lane);
-			for (int c = 0; c < wn; c += 32) {
-				const int q = c + lane;
-				const int64_t p = (int64_t)w0 + q;
-				const uint32_t V = step_bits<4>(win, c, min(32, wn - c));
-				const bool probe = ((V >> lane) & 1u) &&
-						(MODE == SCORE_LENGTH || p >= st.skip_end) &&
-						!dust_low(a.dust[mate], start + (uint64_t)p);
-				const bool hit = probe && contains(F, win.h0[q], reads);
-				const uint32_t H = __ballot_sync(kFull, hit);
-				score_chunk(st, V, H, (int64_t)w0 + c, min(32, wn - c), (int)F.k, a.streak_thr,
-						MODE);
-			}
-			__syncwarp();
-		}
-	}
-	const double v = score_value<MODE>(st, len, F.k, MODE == SCORE_BINOMIAL ? g.sa.fpr[f] : 0.0,
-			lane);
-	if (lane == 0)
-		g.sa.scores[mate][i * a.nf + f] = v;
 }
 
 /* Items of chunk c, reads [32c, 32c + 32), into the warp's queue: those long
@@ -308,21 +118,21 @@ __device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, 
 		l = a.off[mate][i + 1] - o;
 		b = o - a.off_base[mate];
 	}
-	if (in && l < g.k) {
+	if (in && l < g.F.k) {
 		if (SCORE) {
 			ScoreState st;
 			score_init(st);
 			g.sa.scores[mate][i * a.nf + g.f] = MODE == SCORE_BINOMIAL
-					? binomial_score(l, g.k, 0, 0.0, lane) : score_value<MODE>(st, l, g.k, 0.0, lane);
+					? binomial_score(l, g.F.k, 0, 0.0, lane) : score_value<MODE>(st, l, g.F.k, 0.0, lane);
 		} else if (a.nf == 1) {
 			a.hits[mate][i] = 0;
 		}
 	}
-	const bool mine = in && l >= g.k && l <= kLaneMaxBases;
+	const bool mine = in && l >= g.F.k && l <= g.max_bases;
 	const unsigned m = __ballot_sync(kFull, mine);
 	if (mine) {
 		const int q = __popc(m & ((1u << lane) - 1u));
-		const uint32_t frames = (uint32_t)l - g.k + 1u;
+		const uint32_t frames = (uint32_t)l - g.F.k + 1u;
 		w.base[q] = b;
 		w.read[q] = (uint32_t)r;
 		w.len[q] = (uint32_t)l;
@@ -347,22 +157,53 @@ __device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, 
 	return __popc(m);
 }
 
+/* A decision into the read's hit words. */
+__device__ __forceinline__ void lane_write(const LaneArgs &g, uint32_t read, int decided)
+{
+	const ClassifyArgs &a = g.a;
+	const uint32_t mate = read >= a.n ? 1u : 0u;
+	const uint64_t i = read - (mate ? a.n : 0);
+	if (a.nf == 1)
+		a.hits[mate][i] = decided == EVAL_ACCEPT ? 1u : 0u;
+	else if (decided == EVAL_ACCEPT)
+		atomicOr((unsigned long long *)&a.hits[mate][i * a.words + (g.f >> 6)],
+				1ull << (g.f & 63u));
+}
+
+template <bool COUNT>
+__device__ __forceinline__ void lane_count(const ClassifyArgs &a, unsigned long long (&acc)[3],
+		int lane)
+{
+	if (!COUNT)
+		return;
+#pragma unroll
+	for (int j = 0; j < 3; ++j)
+		for (int o = 16; o; o >>= 1)
+			acc[j] += __shfl_xor_sync(kFull, acc[j], o);
+	if (lane == 0) {
+		if (a.probes)
+			atomicAdd(a.probes, acc[0]);
+		if (a.frames)
+			atomicAdd(a.frames, acc[1]);
+		if (a.alg_probes)
+			atomicAdd(a.alg_probes, acc[2]);
+	}
+}
+
 template <int MODE, bool SCORE, bool COUNT, bool PACKED>
 __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 		const __grid_constant__ LaneArgs g)
 {
-	/* per warp: its LaneWarp, or the hash window of a long read before that */
-	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ LaneWarp<MODE> warps[kLaneWarps];
 	__shared__ LaneTables tab;
 	__shared__ double terms[MODE == SCORE_HARMONIC ? kHarmTerms : 1];
 	const ClassifyArgs &a = g.a;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	unsigned char *wmem = smem + warp * lane_warp_bytes<MODE>(a.kmax);
-	LaneWarp<MODE> &w = *reinterpret_cast<LaneWarp<MODE> *>(wmem);
+	LaneWarp<MODE> &w = warps[warp];
 	unsigned long long acc[3] = {0, 0, 0}; /* words read, frames hashed, words of the
 	                                          sequential algorithm */
 	if (warp == 0)
-		lane_tables<PACKED>(tab, g.k, lane);
+		lane_tables<PACKED>(tab, g.F.k, lane);
 	if (MODE == SCORE_HARMONIC && threadIdx.x < kHarmTerms)
 		terms[threadIdx.x] = harmonic_term(threadIdx.x);
 	__syncthreads();
@@ -377,14 +218,18 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			it = __shfl_sync(kFull, it, 0);
 			if (it >= nlong)
 				break;
-			lane_long_item<MODE, SCORE, COUNT>(g, g.list[it], wmem, lane, COUNT ? acc : nullptr);
+			const uint32_t r = g.list[it];
+			const int d = lane_long_item<MODE, SCORE, COUNT, PACKED>(a, &g.sa, g.F, g.f, tab, r,
+					&w.nib[0][0], lane, COUNT ? acc : nullptr);
+			if (!SCORE && lane == 0)
+				lane_write(g, r, d);
 			__syncwarp();
 		}
 	}
 
 	/* the others, a lane each */
-	const int32_t k = (int32_t)g.k;
-	const uint64_t pol = lane_policy(g.keep != 0);
+	const int32_t k = (int32_t)g.F.k;
+	const uint64_t pol = lane_policy(g.F.keep != 0);
 	bool more = true;
 	int qi = 0, qn = 0;         /* queue: next item, items */
 	bool active = false;
@@ -451,15 +296,15 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			const uint32_t mate = w.my_read[lane] >= a.n ? 1u : 0u;
 			uint32_t nib, bad;
 			lane_bases<PACKED>(a, mate, w.my_base[lane] + pos, nb, nib, bad);
-			V = lane_valid(bad, nb, run, g.k);
+			V = lane_valid(bad, nb, run, g.F.k);
 			if (COUNT)
 				acc[1] += __popc(V);
 			/* the bases k before: nibbles from word q8 back, shifted */
-			const uint32_t q8 = (g.k + 7u) >> 3, at = pos >> 3;
+			const uint32_t q8 = (g.F.k + 7u) >> 3, at = pos >> 3;
 			const uint32_t lo = w.nib[(at - q8) & 3u][lane];
 			const uint32_t hi = q8 == 1u ? nib : w.nib[(at - q8 + 1u) & 3u][lane];
 			w.nib[at & 3u][lane] = nib;
-			pairs = nib | (__funnelshift_r(lo, hi, 4u * (8u * q8 - g.k)) << 2);
+			pairs = nib | (__funnelshift_r(lo, hi, 4u * (8u * q8 - g.F.k)) << 2);
 			if (!SCORE) {
 				ev.thres = w.my_thres[lane];
 				ev.anti_thres = w.my_anti_thres[lane];
@@ -495,34 +340,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 						live &= ~(1u << j);
 			}
 			uint32_t cost[COUNT ? kLaneSub : 1];
-			if (COUNT)
-				for (int j = 0; j < kLaneSub; ++j)
-					cost[j] = 0;
-			for (uint32_t i = 0; i < g.h; ++i) {
-				if (!__any_sync(kFull, live != 0u))
-					break;
-				const uint64_t mul = (uint64_t)i ^ g.kmul;
-				uint32_t word[kLaneSub], bit[kLaneSub];
-#pragma unroll
-				for (int j = 0; j < kLaneSub; ++j) {
-					uint64_t v = canon[j];
-					if (i) { /* extra_hash(canon, k, i) */
-						v *= mul;
-						v ^= v >> kMultiShift;
-					}
-					const uint32_t x = lane_word(v, g.m5, g.inv_hi, g.inv_lo);
-					bit[j] = (uint32_t)v;
-					word[j] = 0;
-					if ((live >> j) & 1u)
-						word[j] = lane_probe(g.words + x, pol);
-					if (COUNT)
-						cost[j] += (live >> j) & 1u;
-				}
-				live = 0; /* a frame that was not probed has no word */
-#pragma unroll
-				for (int j = 0; j < kLaneSub; ++j)
-					live += (__funnelshift_r(word[j], word[j], bit[j]) & 1u) * (1u << j);
-			}
+			live = lane_levels<COUNT, kLaneSub>(g.F, canon, live, pol, cost);
 			if (SCORE) {
 				if (Vs)
 					sc.template step<kLaneSub>(Vs, live, p0, k, (int32_t)a.streak_thr, terms);
@@ -551,38 +369,19 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 					const int l = __ffs(m) - 1;
 					const uint32_t hits = __shfl_sync(kFull, (uint32_t)st.score, l);
 					const uint32_t ln = __shfl_sync(kFull, len, l);
-					const double v = binomial_score(ln, g.k, hits, g.sa.fpr[g.f], lane);
+					const double v = binomial_score(ln, g.F.k, hits, g.sa.fpr[g.f], lane);
 					if (lane == l)
 						*out = v;
 				}
 			} else if (done) {
-				*out = score_value<MODE>(st, len, g.k, 0.0, lane);
+				*out = score_value<MODE>(st, len, g.F.k, 0.0, lane);
 			}
 		} else if (done) {
-			const uint32_t read = w.my_read[lane], mate = read >= a.n ? 1u : 0u;
-			const uint64_t i = read - (mate ? a.n : 0);
-			if (a.nf == 1)
-				a.hits[mate][i] = decided == EVAL_ACCEPT ? 1u : 0u;
-			else if (decided == EVAL_ACCEPT)
-				atomicOr((unsigned long long *)&a.hits[mate][i * a.words + (g.f >> 6)],
-						1ull << (g.f & 63u));
+			lane_write(g, w.my_read[lane], decided);
 		}
 		active = active && !done;
 	}
-	if (COUNT) {
-#pragma unroll
-		for (int j = 0; j < 3; ++j)
-			for (int o = 16; o; o >>= 1)
-				acc[j] += __shfl_xor_sync(kFull, acc[j], o);
-		if (lane == 0) {
-			if (a.probes)
-				atomicAdd(a.probes, acc[0]);
-			if (a.frames)
-				atomicAdd(a.frames, acc[1]);
-			if (a.alg_probes)
-				atomicAdd(a.alg_probes, acc[2]);
-		}
-	}
+	lane_count<COUNT>(a, acc, lane);
 }
 
 template <int MODE, bool SCORE, bool COUNT>
@@ -590,17 +389,13 @@ cudaError_t launch_mode(const LaneArgs &g, int num_sms, cudaStream_t s)
 {
 	auto kern = g.a.packed ? lane_kernel<MODE, SCORE, COUNT, true>
 	                       : lane_kernel<MODE, SCORE, COUNT, false>;
-	const size_t smem = kLaneWarps * lane_warp_bytes<MODE>(g.a.kmax);
 	int per_sm = 0;
-	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			(int)smem);
-	if (e == cudaSuccess)
-		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLaneWarps * 32, smem);
+	cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLaneWarps * 32, 0);
 	if (e != cudaSuccess)
 		return e;
 	const uint64_t need = (g.chunks + kLaneWarps - 1) / kLaneWarps;
 	const uint64_t full = (uint64_t)std::max(per_sm, 1) * num_sms;
-	kern<<<(unsigned)std::min(need, full), kLaneWarps * 32, smem, s>>>(g);
+	kern<<<(unsigned)std::min(need, full), kLaneWarps * 32, 0, s>>>(g);
 	return cudaGetLastError();
 }
 
@@ -627,9 +422,23 @@ bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64
 	return true;
 }
 
-bool lane_pays(uint64_t reads)
+/* Whether a filter of the call fits L2. */
+static bool lane_in_l2(const FilterDev *hf, uint32_t nf)
 {
-	return reads >= 8192;
+	for (uint32_t i = 0; i < nf; ++i)
+		if (hf[i].m / 8 <= kLaneKeepBytes)
+			return true;
+	return false;
+}
+
+/* A lane's read takes its time (80 us for 150 bases over a filter in L2, 115-138 us
+ * over one in HBM, whatever the batch's size); the warp kernels' time grows with
+ * the batch and reaches that at about these sizes (reads of 150 bases: 78 us per
+ * 20k reads, 68 per 16k, 106 per 32k in L2; 122 us per 24k, 151 per 32k in HBM; ten filters
+ * of 68 MB: 743 us per 16k reads and 1232 per 32k, against 850). */
+bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads)
+{
+	return total_reads >= (lane_in_l2(hf, nf) ? 20000u : 28000u);
 }
 
 cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreArgs *sa,
@@ -641,12 +450,13 @@ cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreA
 	cudaError_t e = cudaMemsetAsync(ls.ctr, 0, lane_counters(a.nf) * sizeof(unsigned long long), s);
 	if (e != cudaSuccess)
 		return e;
+	LaneArgs g;
+	g.max_bases = lane_in_l2(hf, a.nf) ? kLaneMaxBases : kLaneMaxBasesHbm;
 	const uint64_t need = (total + 255) / 256;
 	lane_long_kernel<<<(unsigned)std::min<uint64_t>(need, (uint64_t)num_sms * 8), 256, 0, s>>>(a,
-			ls.list, ls.ctr);
+			g.max_bases, ls.list, ls.ctr);
 	if ((e = cudaGetLastError()) != cudaSuccess)
 		return e;
-	LaneArgs g;
 	g.a = a;
 	g.sa = sa ? *sa : ScoreArgs();
 	g.list = ls.list;
@@ -654,16 +464,7 @@ cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreA
 	g.chunks = (total + 31) / 32;
 	g.ctr = ls.ctr + 1;
 	for (g.f = 0; g.f < a.nf; ++g.f, g.ctr += 2) {
-		const FilterDev &F = hf[g.f];
-		g.k = F.k;
-		g.h = F.h;
-		g.kmul = F.kmul;
-		g.words = F.words;
-		g.keep = F.m / 8 <= kLaneKeepBytes;
-		g.m5 = (uint32_t)(F.m >> 5);
-		const uint64_t inv = ~0ull / g.m5;
-		g.inv_hi = (uint32_t)(inv >> 32);
-		g.inv_lo = (uint32_t)inv;
+		g.F = lane_filter(hf[g.f]);
 		e = sa ? launch_lane_as<true, false>(g, num_sms, s)
 		  : count ? launch_lane_as<false, true>(g, num_sms, s)
 		          : launch_lane_as<false, false>(g, num_sms, s);

@@ -18,10 +18,10 @@ struct LaneScratch {
 	unsigned long long *ctr;
 };
 
-/* Whether the lane kernel takes these filters and options; lane_pays says from
- * which number of reads on it should. */
+/* Whether the lane kernel takes these filters and options, and whether it is the
+ * faster one for a batch of so many reads. */
 bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64_t total_reads);
-bool lane_pays(uint64_t reads);
+bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads);
 
 /* Counters of a launch (which is a kernel per filter, after one that lists long
  * reads). */

@@ -1,4 +1,4 @@
-"""The lane kernel (batches of at least 8192 reads): hits, probe
+"""The lane kernel (batches of at least 20,000 reads, over filters that fit L2): hits, probe
 counts, categories and scores against the oracle, for ASCII and packed bases at
 any offset, reads and pairs, filters of one and of several k, every scoring
 method, masking, reads around the length from which a warp takes a read, a
@@ -102,7 +102,7 @@ def test_hits_and_probe_counts(tmp_path, ks, h, scoring, score, streak, paired, 
     import torch
     rng = np.random.default_rng(len(ks) * 1000 + ks[0] * 10 + scoring)
     genomes, filters, paths = _filters(tmp_path, rng, ks, h)
-    n = 8200 // (2 if paired else 1) + 37
+    n = 28100 // (2 if paired else 1) + 37
     mates = [_reads(rng, genomes, n, ks[0]) for _ in range(2 if paired else 1)]
     thr = 10.0 ** (-score / 10.0) if scoring == ol.BINOMIAL else score
     want, alg = [], 0
@@ -136,7 +136,7 @@ def test_packed_bases(tmp_path, ks, h, lead, with_valid):
     from biobloom_b200 import _lib as L
     rng = np.random.default_rng(50 + lead)
     genomes, filters, paths = _filters(tmp_path, rng, ks, h)
-    reads = _reads(rng, genomes, 8300, ks[0])
+    reads = _reads(rng, genomes, 20300, ks[0])
     if not with_valid:
         reads = [bytes(c if c in b"ACGTacgt" else 65 for c in r) for r in reads]
     seq, off = ol.pack_reads(reads)
@@ -173,7 +173,7 @@ def test_scores_and_best_hits(tmp_path, ks, scoring, paired):
     from biobloom_b200 import MODE_BESTHIT, MODE_SCORES
     rng = np.random.default_rng(70 + scoring + len(ks))
     genomes, filters, paths = _filters(tmp_path, rng, ks, 3)
-    n = 8200 // (2 if paired else 1) + 11
+    n = 20100 // (2 if paired else 1) + 11
     mates = [_reads(rng, genomes, n, ks[0]) for _ in range(2 if paired else 1)]
     want = [ol.classify_scores(*ol.pack_reads(m), filters, scoring, 3) for m in mates]
     score = {ol.LENGTH: 40, ol.BINOMIAL: 100}.get(scoring, 0.15)
@@ -203,7 +203,7 @@ def test_dust_and_ordered(tmp_path):
     from biobloom_b200 import MODE_ORDERED
     rng = np.random.default_rng(90)
     genomes, filters, paths = _filters(tmp_path, rng, [25, 25, 25], 3)
-    reads = _reads(rng, genomes, 8400, 25)
+    reads = _reads(rng, genomes, 20400, 25)
     with ol.dust():
         want, _ = ol.classify(*ol.pack_reads(reads), filters, 0.15, 3)
     with _open(paths, ol.SIMPLE, 0.15, 3) as bbc:
@@ -224,10 +224,10 @@ def test_graph_replays_on_new_reads(tmp_path):
     import torch
     rng = np.random.default_rng(91)
     genomes, filters, paths = _filters(tmp_path, rng, [25], 3)
-    a, b = _reads(rng, genomes, 9000, 25), _reads(rng, genomes, 9000, 25)
+    a, b = _reads(rng, genomes, 20900, 25), _reads(rng, genomes, 20900, 25)
     (sa, oa), (sb, ob) = _device(a), _device(b)
     seq = torch.zeros(max(len(sa), len(sb)), dtype=torch.uint8, device="cuda")
-    off, hits = oa.clone(), torch.empty((9000, 1), dtype=torch.int64, device="cuda")
+    off, hits = oa.clone(), torch.empty((20900, 1), dtype=torch.int64, device="cuda")
     stream = torch.cuda.Stream()
     with _open(paths, ol.SIMPLE, 0.15, 3) as bbc:
         g = bbc.graph(seq, off, hits)
@@ -241,3 +241,33 @@ def test_graph_replays_on_new_reads(tmp_path):
             want, _ = ol.classify(*ol.pack_reads(reads), filters, 0.15, 3)
             assert np.array_equal(hits.cpu().numpy().view(np.uint64), want)
         g.close()
+
+
+@pytest.mark.parametrize("ks,h,scoring,score,streak,paired,lead", CASES)
+def test_long_reads_of_small_batches(tmp_path, ks, h, scoring, score, streak, paired, lead):
+    """Below that size the warp kernel takes the batch, and evaluates reads above
+    384 bases in windows of 256 frames."""
+    import torch
+    rng = np.random.default_rng(ks[0] * 10 + scoring)
+    genomes, filters, paths = _filters(tmp_path, rng, ks, h)
+    mates = [_reads(rng, genomes, 300, ks[0]) + _reads(rng, genomes, 60, ks[0])
+             for _ in range(2 if paired else 1)]
+    for m in mates:
+        for n in (383, 384, 385, 256 + ks[0] - 1, 512 + ks[0] - 1, 512 + ks[0], 6000):
+            st = int(rng.integers(0, 20000 - n))
+            m[int(rng.integers(0, 300))] = genomes[0][st:st + n].tobytes()
+            m[int(rng.integers(0, 300))] = rng.choice(ACGT, n).tobytes()
+    thr = 10.0 ** (-score / 10.0) if scoring == ol.BINOMIAL else score
+    with _open(paths, scoring, score, streak, path=2) as bbc:
+        dev = [t for m in mates for t in _device(m, lead)]
+        for count in (False, True):
+            bbc.set_counting(count)
+            got = bbc.classify_device(*dev)
+            torch.cuda.synchronize()
+            alg = 0
+            for m, t in zip(mates, (got[0], got[1])):
+                w, a = ol.classify(*ol.pack_reads(m), filters, thr, streak, scoring=scoring,
+                                   count_probes=True)
+                alg += a
+                assert np.array_equal(t.cpu().numpy().view(np.uint64), w)
+        assert bbc.last_stats()["probes_algorithmic"] == alg
