@@ -42,6 +42,7 @@
 
 #include "bbt_device.cuh"
 #include "bucketed.cuh"
+#include "lane_item.cuh"
 #include "mibf_ctx.hpp"
 #include "window.cuh"
 
@@ -51,6 +52,7 @@ constexpr int kBlockBits = 224;
 constexpr int kSuperShift = 20;
 constexpr int kStageBases = 512;
 constexpr int kReadsPerGrab = 4;
+constexpr size_t kFrameCountWords = 1 + 2048 + 1; /* mibf_frame_counts_kernel */
 
 struct MibfDev {
 	const uint4 *blocks;
@@ -665,6 +667,8 @@ __global__ void __launch_bounds__(kQueryThreads, kQueryMinBlocks) mibf_query_ker
 	}
 }
 
+#include "mibf_scan.cuh"
+
 /* Add a batch's summary counters to the context's, unless a read of the
  * batch overflowed its result slots (the caller then runs the batch again). */
 __global__ void mibf_commit_kernel(const unsigned long long *batch, unsigned long long *total,
@@ -679,20 +683,45 @@ __global__ void mibf_commit_kernel(const unsigned long long *batch, unsigned lon
 		atomicAdd(total + n, (unsigned long long)reads);
 }
 
-/* Largest frame count of a device batch and a bitmap of the frame counts
- * below 65536 that occur. */
-__global__ void mibf_frame_counts_kernel(const uint64_t *off, const uint64_t *off2, uint64_t n,
-		uint32_t k, unsigned int *out)
+/* Largest frame count of a device batch, a bitmap of the frame counts below
+ * 65536 that occur and, last, the most frames of a read (pair).  A block
+ * collects its reads' in shared memory: reads of one length would otherwise
+ * all take turns at the same two words (340 us per 500k reads; now 6). */
+__global__ void __launch_bounds__(256) mibf_frame_counts_kernel(const uint64_t *off,
+		const uint64_t *off2, uint64_t n, uint32_t k, unsigned int *out)
 {
+	__shared__ unsigned int seen[2048], most, total;
+	for (uint32_t i = threadIdx.x; i < 2048; i += blockDim.x)
+		seen[i] = 0;
+	if (threadIdx.x == 0)
+		most = total = 0;
+	__syncthreads();
+	uint32_t mine = 0, mine_total = 0;
 	for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < n;
 			r += (uint64_t)gridDim.x * blockDim.x) {
 		const uint64_t l1 = off[r + 1] - off[r];
 		const uint64_t l2 = off2 ? off2[r + 1] - off2[r] : 0;
-		const uint64_t f64 = l1 >= k ? l1 - k + 1 : (l2 >= k ? l2 - k + 1 : 0);
+		const uint64_t f1 = l1 >= k ? l1 - k + 1 : 0, f2 = l2 >= k ? l2 - k + 1 : 0;
+		const uint64_t f64 = f1 ? f1 : f2;
 		const uint32_t fc = f64 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)f64;
-		atomicMax(out, fc);
-		if (fc < 65536u)
-			atomicOr(out + 1 + (fc >> 5), 1u << (fc & 31));
+		mine = max(mine, fc);
+		mine_total = max(mine_total, f1 + f2 > 0xFFFFFFFFull ? 0xFFFFFFFFu : (uint32_t)(f1 + f2));
+		if (fc < 65536u && !((*(volatile unsigned int *)&seen[fc >> 5] >> (fc & 31)) & 1u))
+			atomicOr(&seen[fc >> 5], 1u << (fc & 31));
+	}
+	mine = __reduce_max_sync(kFull, mine);
+	mine_total = __reduce_max_sync(kFull, mine_total);
+	if ((threadIdx.x & 31) == 0) {
+		atomicMax(&most, mine);
+		atomicMax(&total, mine_total);
+	}
+	__syncthreads();
+	for (uint32_t i = threadIdx.x; i < 2048; i += blockDim.x)
+		if (seen[i])
+			atomicOr(out + 1 + i, seen[i]);
+	if (threadIdx.x == 0) {
+		atomicMax(out, most);
+		atomicMax(out + 1 + 2048, total);
 	}
 }
 
@@ -1522,7 +1551,7 @@ extern "C" int bbt_mibf_open(const char *bf_path, const bbt_mibf_params *params,
 			cudaMalloc(&ctx->d_work, 8) != cudaSuccess ||
 			cudaMalloc(&ctx->d_flags, 4) != cudaSuccess ||
 			cudaMalloc(&ctx->d_stat, 3 * 8) != cudaSuccess ||
-			cudaMalloc(&ctx->d_fcmax, (1 + 2048) * 4) != cudaSuccess)
+			cudaMalloc(&ctx->d_fcmax, kFrameCountWords * 4) != cudaSuccess)
 		return bail(mibf_fail(ctx, BBT_ERR_NOMEM, "cudaMalloc(context)"));
 	cudaMemcpy(ctx->d_tables, tabs.data(), tabs.size() * 8, cudaMemcpyHostToDevice);
 	cudaMemset(ctx->d_counts, 0, 2 * nc * 8);
@@ -1560,8 +1589,14 @@ static int ensure_min_count(bbt_mibf *ctx, const std::vector<uint32_t> &fcs, cud
 		ctx->h_minc[(size_t)fc * nids + id] = id == 0 ? 0u
 				: mibf_min_count(fc, ctx->frame_prob[id], ctx->p.score, nids);
 	}
-	for (uint32_t fc : missing)
+	for (uint32_t fc : missing) {
+		/* entry 0 (no ID): the smallest of the row */
+		uint32_t *row = &ctx->h_minc[(size_t)fc * nids];
+		row[0] = ~0u;
+		for (unsigned id = 1; id < nids; ++id)
+			row[0] = std::min(row[0], row[id]);
 		ctx->minc_have[fc] = 1;
+	}
 	if (ctx->minc_rows < need_rows) {
 		uint32_t rows = std::max<uint32_t>(need_rows, ctx->minc_rows * 2);
 		rows = std::max<uint32_t>(rows, 256);
@@ -1644,17 +1679,30 @@ static std::vector<uint32_t> host_frame_counts(const bbt_batch *b, unsigned k)
 	return fcs;
 }
 
-static int device_frame_counts(bbt_mibf *ctx, const bbt_batch *b, cudaStream_t s,
-		std::vector<uint32_t> &fcs)
+uint64_t bbt::mibf_most_frames(const bbt_mibf *ctx, const uint64_t *off, const uint64_t *off2,
+		uint64_t n)
 {
-	MIBF_TRY(ctx, cudaMemsetAsync(ctx->d_fcmax, 0, (1 + 2048) * 4, s));
+	const uint64_t k = ctx->hd.k;
+	uint64_t most = 0;
+	for (uint64_t r = 0; r < n; ++r) {
+		const uint64_t l1 = off[r + 1] - off[r], l2 = off2 ? off2[r + 1] - off2[r] : 0;
+		most = std::max(most, (l1 >= k ? l1 - k + 1 : 0) + (l2 >= k ? l2 - k + 1 : 0));
+	}
+	return most;
+}
+
+static int device_frame_counts(bbt_mibf *ctx, const bbt_batch *b, cudaStream_t s,
+		std::vector<uint32_t> &fcs, uint64_t &most)
+{
+	MIBF_TRY(ctx, cudaMemsetAsync(ctx->d_fcmax, 0, kFrameCountWords * 4, s));
 	mibf_frame_counts_kernel<<<ctx->num_sms * 4, 256, 0, s>>>(b->offsets,
 			b->seq2 ? b->offsets2 : nullptr, b->n_reads, ctx->hd.k, ctx->d_fcmax);
-	std::vector<unsigned int> h(1 + 2048);
+	std::vector<unsigned int> h(kFrameCountWords);
 	MIBF_TRY(ctx, cudaMemcpyAsync(h.data(), ctx->d_fcmax, h.size() * 4, cudaMemcpyDeviceToHost,
 			s));
 	MIBF_TRY(ctx, cudaStreamSynchronize(s));
 	const uint32_t mx = h[0];
+	most = h[1 + 2048];
 	for (uint32_t fc = 0; fc < 65536 && fc <= mx; ++fc)
 		if ((h[1 + (fc >> 5)] >> (fc & 31)) & 1u)
 			fcs.push_back(fc);
@@ -1883,6 +1931,54 @@ static int run_query_bucketed(bbt_mibf *ctx, const MibfArgs &a, int hsel, bool b
 	return BBT_OK;
 }
 
+/* Whether reads of up to most_frames frames (both mates) take mibf_scan_kernel:
+ * the dense map, IDs in shared memory, 16-bit counters, up to 8 values a frame.
+ * It is the faster one wherever both run (500k reads against 500 targets: 7.2 ->
+ * 4.1 ms; 50k ragged pairs against 100: 1.6 -> 0.8). */
+static bool scan_takes(const bbt_mibf *ctx, uint64_t most_frames)
+{
+	return ctx->d_dense && !big_ids(ctx) && ctx->hd.h <= 8 && (ctx->hd.m >> 5) < (1ull << 30) &&
+			most_frames * ctx->hd.h < 65536;
+}
+
+template <int H>
+static cudaError_t launch_scan_h(const MibfArgs &a, const ScanLists &l, int num_sms, cudaStream_t s)
+{
+	const size_t smem = scan_smem(a.f.nids);
+	cudaError_t e = cudaFuncSetAttribute(mibf_scan_kernel<H>,
+			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	int nb = 0;
+	if (e == cudaSuccess)
+		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mibf_scan_kernel<H>, kScanThreads,
+				smem);
+	if (e != cudaSuccess)
+		return e;
+	/* probes on their way need room in L1: blocks only while they leave it 88 of
+	 * the SM's 228 KB, and no more shared memory carved out than they use (500
+	 * targets, 68 KB a block: 5.6 ms at three blocks per SM, 4.1 at two) */
+	nb = std::max(1, std::min(nb, (int)(kScanSmemPerSm / (smem + 1024))));
+	e = cudaFuncSetAttribute(mibf_scan_kernel<H>, cudaFuncAttributePreferredSharedMemoryCarveout,
+			(int)std::min<size_t>(100, (nb * (smem + 1024) * 100 + (228 << 10) - 1) / (228 << 10)));
+	if (e != cudaSuccess)
+		return e;
+	const uint64_t need = (a.n_reads + kScanThreads / 32 - 1) / (kScanThreads / 32);
+	const uint64_t full = (uint64_t)nb * num_sms;
+	mibf_scan_kernel<H><<<(unsigned)std::min(need, full), kScanThreads, smem, s>>>(a, l);
+	return cudaGetLastError();
+}
+
+static cudaError_t launch_scan(const MibfArgs &a, const ScanLists &l, int num_sms, cudaStream_t s)
+{
+	switch (pick_h(a.f.h)) {
+	case 1: return launch_scan_h<1>(a, l, num_sms, s);
+	case 2: return launch_scan_h<2>(a, l, num_sms, s);
+	case 3: return launch_scan_h<3>(a, l, num_sms, s);
+	case 4: return launch_scan_h<4>(a, l, num_sms, s);
+	case 6: return launch_scan_h<6>(a, l, num_sms, s);
+	default: return launch_scan_h<8>(a, l, num_sms, s);
+	}
+}
+
 /* A batch may be classified in several launches (chunks of its reads, their
  * results at their place in the batch's arrays): the first clears the batch's
  * counters and overflow flag, the last commits the counters. */
@@ -1898,7 +1994,7 @@ struct MibfEncoding {
 static int run_query_sc(bbt_mibf *ctx, uint64_t n_reads, const uint8_t *seq, const uint64_t *off,
 		const uint8_t *seq2, const uint64_t *off2, bbt_mibf_hit *hits, uint32_t max_hits,
 		uint32_t *n_hits, uint32_t *sat, cudaStream_t s, const MibfScratch &sc, bool timed,
-		int phase = kQueryWhole, uint64_t total_reads = ~0ull, MibfEncoding enc = MibfEncoding())
+		uint64_t most_frames, int phase = kQueryWhole, uint64_t total_reads = ~0ull, MibfEncoding enc = MibfEncoding())
 {
 	if (total_reads == ~0ull)
 		total_reads = n_reads;
@@ -1969,7 +2065,9 @@ static int run_query_sc(bbt_mibf *ctx, uint64_t n_reads, const uint8_t *seq, con
 	}
 	if (!bucketed) {
 		MIBF_TRY(ctx, cudaMemsetAsync(sc.work, 0, 8, s));
-		if (n_reads)
+		if (n_reads && scan_takes(ctx, most_frames))
+			MIBF_TRY(ctx, launch_scan(a, scan_lists(ctx->hd.seeds, ctx->hd.k), ctx->num_sms, s));
+		else if (n_reads)
 			MIBF_TRY(ctx, launch_query(a, dense, big, hsel, grid, smem, s));
 	}
 	if (phase & kQueryEnd) {
@@ -2008,10 +2106,10 @@ static MibfEncoding batch_encoding(const bbt_batch *b)
 
 static int run_query(bbt_mibf *ctx, const bbt_batch *b, const uint8_t *seq, const uint64_t *off,
 		const uint8_t *seq2, const uint64_t *off2, bbt_mibf_hit *hits, uint32_t max_hits,
-		uint32_t *n_hits, uint32_t *sat, cudaStream_t s)
+		uint32_t *n_hits, uint32_t *sat, cudaStream_t s, uint64_t most_frames)
 {
 	return run_query_sc(ctx, b->n_reads, seq, off, seq2, off2, hits, max_hits, n_hits, sat, s,
-			ctx_scratch(ctx), true, kQueryWhole, ~0ull, batch_encoding(b));
+			ctx_scratch(ctx), true, most_frames, kQueryWhole, ~0ull, batch_encoding(b));
 }
 
 int bbt::mibf_scratch_init(bbt_mibf *ctx, MibfScratch &sc)
@@ -2040,9 +2138,10 @@ void bbt::mibf_scratch_free(MibfScratch &sc)
 
 int bbt::mibf_classify_slot(bbt_mibf *ctx, uint64_t n, const uint8_t *seq, const uint64_t *off,
 		const uint8_t *seq2, const uint64_t *off2, bbt_mibf_hit *hits, uint32_t max_hits,
-		uint32_t *n_hits, uint32_t *sat, cudaStream_t s, MibfScratch &sc)
+		uint32_t *n_hits, uint32_t *sat, uint64_t most_frames, cudaStream_t s, MibfScratch &sc)
 {
-	return run_query_sc(ctx, n, seq, off, seq2, off2, hits, max_hits, n_hits, sat, s, sc, false);
+	return run_query_sc(ctx, n, seq, off, seq2, off2, hits, max_hits, n_hits, sat, s, sc, false,
+			most_frames);
 }
 
 /* Chunk slots of the host-batch pipeline, for chunks of up to `reads` reads
@@ -2096,7 +2195,7 @@ constexpr uint64_t kChunkBases = 256ull << 20;
  * overflowed max_hits), so results and summary equal one launch's.
  */
 static int classify_host_chunks(bbt_mibf *ctx, const bbt_batch *b, bbt_mibf_result *res,
-		cudaStream_t s)
+		cudaStream_t s, uint64_t most_frames)
 {
 	const uint64_t n = b->n_reads;
 	if (n == 0) {
@@ -2206,7 +2305,7 @@ static int classify_host_chunks(bbt_mibf *ctx, const bbt_batch *b, bbt_mibf_resu
 		rc = run_query_sc(ctx, cnt, ctx->c_seq[sl][0], ctx->c_off[sl][0],
 				paired ? ctx->c_seq[sl][1] : nullptr, paired ? ctx->c_off[sl][1] : nullptr,
 				ctx->d_hits + r0 * res->max_hits, res->max_hits, ctx->d_nhits + r0,
-				ctx->d_sat + r0, s, sc, true, phase, n, enc);
+				ctx->d_sat + r0, s, sc, true, most_frames, phase, n, enc);
 		if (rc)
 			return rc;
 		MIBF_TRY(ctx, cudaEventRecord(ctx->c_computed[sl], s));
@@ -2254,20 +2353,22 @@ extern "C" int bbt_mibf_classify_batch(bbt_mibf *ctx, const bbt_batch *b, bbt_mi
 	int rc;
 	if (b->location == BBT_DEVICE) {
 		std::vector<uint32_t> fcs;
-		rc = device_frame_counts(ctx, b, s, fcs);
+		uint64_t most = 0;
+		rc = device_frame_counts(ctx, b, s, fcs, most);
 		if (rc)
 			return rc;
 		rc = ensure_min_count(ctx, fcs, s);
 		if (rc)
 			return rc;
 		return run_query(ctx, b, (const uint8_t *)b->seq, b->offsets, (const uint8_t *)b->seq2,
-				b->offsets2, res->hits, res->max_hits, res->n_hits, res->sat_count, s);
+				b->offsets2, res->hits, res->max_hits, res->n_hits, res->sat_count, s, most);
 	}
 	/* host batch: chunks through two slots, copies overlapping the launches */
 	rc = ensure_min_count(ctx, host_frame_counts(b, ctx->hd.k), s);
 	if (rc)
 		return rc;
-	return classify_host_chunks(ctx, b, res, s);
+	return classify_host_chunks(ctx, b, res, s,
+			mibf_most_frames(ctx, b->offsets, b->seq2 ? b->offsets2 : nullptr, b->n_reads));
 }
 
 extern "C" int bbt_mibf_sync(bbt_mibf *ctx)

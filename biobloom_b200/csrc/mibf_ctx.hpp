@@ -168,10 +168,14 @@ int mibf_reserve_rows(bbt_mibf *ctx, uint32_t rows);
 int mibf_rows_for(bbt_mibf *ctx, const uint64_t *off, const uint64_t *off2, uint64_t n);
 /* Classify n reads (pairs) on the device on stream s with this scratch; the
  * batch's summary is committed unless a read overflowed max_hits, which sets
- * sc.flags[0] (read it after the stream completes). */
+ * sc.flags[0] (read it after the stream completes).  most_frames:
+ * mibf_most_frames of the reads, or more. */
 int mibf_classify_slot(bbt_mibf *ctx, uint64_t n, const uint8_t *seq, const uint64_t *off,
 		const uint8_t *seq2, const uint64_t *off2, bbt_mibf_hit *hits, uint32_t max_hits,
-		uint32_t *n_hits, uint32_t *sat, cudaStream_t s, MibfScratch &sc);
+		uint32_t *n_hits, uint32_t *sat, uint64_t most_frames, cudaStream_t s, MibfScratch &sc);
+/* Frames of the read (pair) that has the most (host offsets). */
+uint64_t mibf_most_frames(const bbt_mibf *ctx, const uint64_t *off, const uint64_t *off2,
+		uint64_t n);
 /* load the header, IDs file names, ID array (host) and frame probabilities */
 int mibf_load_host(bbt_mibf *ctx, const char *bf_path, std::vector<uint16_t> *ids_out);
 }

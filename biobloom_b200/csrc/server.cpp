@@ -249,7 +249,8 @@ int run_chunk(bbt_server *srv, ServeSlot &sl, Req &q, char *base, uint64_t i0, u
 		uint32_t *dn = (uint32_t *)(base + L.out[1]);
 		uint32_t *ds = (uint32_t *)(base + L.out[2]);
 		rc = mibf_classify_slot(srv->mi, c, dseq[0], doff[0], dseq[1], doff[1], dh,
-				r.mi_max_hits, dn, ds, s, sl.mi);
+				r.mi_max_hits, dn, ds, mibf_most_frames(srv->mi, sl.h_off,
+				paired ? sl.h_off + srv->p.chunk_reads + 1 : nullptr, c), s, sl.mi);
 		if (rc)
 			return rc;
 		if (r.mi_hits && r.mi_max_hits && cudaMemcpyAsync(r.mi_hits + i0 * mh, dh,
