@@ -1167,14 +1167,17 @@ static int run_dust(bbt_ctx *ctx, ClassifyArgs &a, const uint64_t *mate_bases, c
 		d.off_base[m] = a.off_base[m];
 		d.mask[m] = ctx->d_dust[m];
 	}
-	int rc = grow(ctx, &ctx->d_dust_redo, ctx->dust_redo_cap, a.n * a.mates);
+	int rc = grow(ctx, &ctx->d_dust_redo, ctx->dust_redo_cap, 2 * a.n * a.mates);
 	if (rc)
 		return rc;
 	CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_dust_cnt, 0, sizeof(unsigned long long), s));
+	CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_dust_cnt + 2, 0, sizeof(unsigned long long), s));
 	d.n = a.n;
 	d.mates = a.mates;
 	d.T = ctx->dust_T;
 	d.W = ctx->dust_W;
+	d.todo = ctx->d_dust_redo + a.n * a.mates;
+	d.todo_count = ctx->d_dust_cnt + 2;
 	d.redo = ctx->d_dust_redo;
 	d.redo_count = ctx->d_dust_cnt;
 	d.failed = ctx->d_dust_cnt + 1;
@@ -1184,7 +1187,7 @@ static int run_dust(bbt_ctx *ctx, ClassifyArgs &a, const uint64_t *mate_bases, c
 	CUDA_TRY(ctx, launch_dust_pass2(d, ctx->dust_threads2, s));
 	a.dust[0] = ctx->d_dust[0];
 	a.dust[1] = a.mates == 2 ? ctx->d_dust[1] : nullptr;
-	ctx->last.kernels += 2;
+	ctx->last.kernels += 3;
 	return BBT_OK;
 }
 
@@ -1808,7 +1811,7 @@ static int set_dust_one(bbt_ctx *ctx, int on, unsigned T, unsigned W)
 		ctx->dust_threads2 = (uint32_t)threads;
 	}
 	if (!ctx->d_dust_cnt)
-		CUDA_TRY(ctx, cudaMalloc(&ctx->d_dust_cnt, 2 * sizeof(unsigned long long)));
+		CUDA_TRY(ctx, cudaMalloc(&ctx->d_dust_cnt, 3 * sizeof(unsigned long long)));
 	ctx->dust = true;
 	ctx->dust_T = (int)T;
 	ctx->dust_W = (int)W;

@@ -81,9 +81,10 @@ struct bbt_ctx {
 	int dust_T = 20, dust_W = 64;
 	uint32_t *d_dust[2] = {nullptr, nullptr};  /* per-mate masked-base bits */
 	uint64_t dust_words_cap[2] = {0, 0};
-	uint64_t *d_dust_redo = nullptr;
+	uint64_t *d_dust_redo = nullptr; /* reads for pass 2, then those of the full scan */
 	uint64_t dust_redo_cap = 0;
-	unsigned long long *d_dust_cnt = nullptr;  /* reads queued for pass 2, reads failed */
+	unsigned long long *d_dust_cnt = nullptr;  /* reads queued for pass 2, reads failed,
+	                                               reads of the full scan */
 	void *d_dust_scratch = nullptr;
 	uint64_t dust_per_thread = 0;
 	uint32_t dust_threads2 = 0;

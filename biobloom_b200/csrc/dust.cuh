@@ -27,6 +27,8 @@ struct DustArgs {
 	uint32_t mates;
 	int T, W;
 	uint32_t *mask[2];
+	uint64_t *todo;                  /* n * mates entries: reads of the full scan */
+	unsigned long long *todo_count;  /* zeroed */
 	uint64_t *redo;
 	unsigned long long *redo_count;
 	unsigned long long *failed;
@@ -35,8 +37,9 @@ struct DustArgs {
 };
 
 size_t dust_perfect_bytes();
-/* Pass 1: every read; reads whose perfect list outgrows the thread's own
- * array are appended to redo. */
+/* Passes 0 and 1: the reads that may hold a masked interval, then those in
+ * full; reads whose perfect list outgrows the thread's own array are appended to
+ * redo. */
 cudaError_t launch_dust_pass1(const DustArgs &a, int num_sms, cudaStream_t s);
 /* Pass 2: the reads pass 1 queued (their count is read on the device), on
  * `threads` threads (a multiple of 32) with scratch_per_thread entries

@@ -26,15 +26,73 @@ struct DustPerfect {
 	int start, finish, r, l;
 };
 
+/* A, C, G, T (either case): 0 to 3; any other byte: 4.  Bits 1 and 2 tell the
+ * four apart (A, C, T, G in that order), without a branch. */
 BBT_DHD int dust_code(uint8_t c)
 {
-	switch (c) {
-	case 'A': case 'a': return 0;
-	case 'C': case 'c': return 1;
-	case 'G': case 'g': return 2;
-	case 'T': case 't': return 3;
-	default: return 4;
+	const unsigned u = c & 0xDFu, v = (u >> 1) & 3u;
+	return ((0x47544341u >> (8u * v)) & 0xFFu) == u ? (int)(v ^ (v >> 1)) : 4;
+}
+
+/* Whether sdust over the read would ever look for perfect intervals (a read for
+ * which it does not has nothing masked): the window's score and the length of
+ * its suffix of dust_scan alone.  The suffix starts after the (m + 1)-th latest
+ * occurrence, m = T / 5, of whichever kind has so many; each window entry
+ * holds its distance to the one of its kind before, so that the start takes m
+ * steps where dust_scan removes the entries up to it one by one.
+ * kind(t): a 32-bit word per triplet kind (its count in the window, and its
+ * latest entry's number above), zero before; ring(i): entry i of W - 2, 16 bits
+ * (kind, distance above). */
+template <class SeqFn, class KindFn, class RingFn>
+BBT_DHD bool dust_may_mask(SeqFn &&seq, uint64_t len, int T, int W, KindFn &&kind, RingFn &&ring)
+{
+	const int cap = W - 2, n = (int)len, m = T / 5;
+	int rw = 0, head = 0, size = 0, l = 0;
+	int p = 0, start = 0; /* next entry's number, first one of the suffix */
+	unsigned t = 0;
+	for (int i = 0; i < n; ++i) {
+		const int b = dust_code(seq(i));
+		if (b >= 4) {
+			l = 0;
+			t = 0;
+			continue;
+		}
+		++l;
+		t = (t << 2 | (unsigned)b) & 63u;
+		if (l < 3)
+			continue;
+		/* the slot of entry p is that of entry p - cap */
+		if (size >= cap) {
+			uint32_t &c = kind(ring(head) & 63u);
+			--c;
+			rw -= (int)(c & 0xFFFFu);
+			--size;
+		}
+		uint32_t &c = kind(t);
+		const unsigned back = ((unsigned)p - (c >> 16)) & 0xFFFFu;
+		rw += (int)(c & 0xFFFFu);
+		c = ((unsigned)p << 16) | ((c & 0xFFFFu) + 1u);
+		ring(head) = (uint16_t)(t | (back & 1023u) << 6);
+		++size;
+		if (start <= p - size)
+			start = p - size + 1;
+		if ((int)(c & 0xFFFFu) > m) {
+			int q = p, at = head;
+			for (int j = 0; j < m; ++j) {
+				const int d = (int)(ring(at) >> 6);
+				q -= d;
+				at -= d;
+				at = at < 0 ? at + cap : at;
+			}
+			if (start <= q)
+				start = q + 1;
+		}
+		++p;
+		head = head + 1 == cap ? 0 : head + 1;
+		if (rw * 10 > (p - start) * T)
+			return true;
 	}
+	return false;
 }
 
 /* sdust over one read; false when the perfect list would exceed pcap
@@ -43,7 +101,7 @@ template <class SeqFn, class MaskFn>
 BBT_DHD bool dust_scan(SeqFn &&seq, uint64_t len, int T, int W, DustPerfect *perf,
 		int pcap, uint8_t *ring, MaskFn &&mask)
 {
-	uint16_t cw[64], cv[64];
+	alignas(16) uint16_t cw[64], cv[64];
 	for (int i = 0; i < 64; ++i)
 		cw[i] = cv[i] = 0;
 	int rw = 0, rv = 0, L = 0;
@@ -125,9 +183,15 @@ BBT_DHD bool dust_scan(SeqFn &&seq, uint64_t len, int T, int W, DustPerfect *per
 			 * entries go to the top of the array (downwards) and are merged in
 			 * after the scan at the positions the reference inserts them:
 			 * after every older entry whose start is not smaller. */
-			uint16_t c[64];
+			alignas(16) uint16_t c[64];
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+			for (int q = 0; q < 8; ++q)
+				reinterpret_cast<uint4 *>(c)[q] = reinterpret_cast<const uint4 *>(cv)[q];
+#else
 			for (int q = 0; q < 64; ++q)
 				c[q] = cv[q];
+#endif
 			int r = rv, max_r = 0, max_l = 0;
 			int jp = 0, nn = 0;
 			for (int k = size - L - 1; k >= 0; --k) {
