@@ -1220,15 +1220,19 @@ static int run_lane(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreAr
 		bool classify)
 {
 	const LaneScratch ls = {ctx->d_lane_list, ctx->d_order_cnt};
+	const bool count = ctx->lc.count != 0;
+	const bool both = classify && sa && !count; /* one walk for hits and scores */
 	if (classify) {
 		const size_t hb = a.n * ctx->words * sizeof(uint64_t);
 		for (uint32_t m = 0; ctx->nf > 1 && m < a.mates; ++m)
 			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
-		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, ls, ctx->num_sms, ctx->lc.count != 0, s));
+	}
+	if (classify && !both) {
+		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, true, ls, ctx->num_sms, count, s));
 		ctx->last.kernels += 1 + ctx->nf;
 	}
 	if (sa) {
-		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), sa, ls, ctx->num_sms, false, s));
+		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), sa, both, ls, ctx->num_sms, false, s));
 		ctx->last.kernels += 1 + ctx->nf;
 	}
 	return BBT_OK;
@@ -2409,7 +2413,7 @@ int bbt::bf_classify_slot(bbt_ctx *ctx, const uint8_t *seq, const uint64_t *off,
 		for (uint32_t m = 0; ctx->nf > 1 && m < a.mates; ++m)
 			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
 		const LaneScratch ls = {reinterpret_cast<uint32_t *>(sc.order), sc.order_cnt};
-		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, ls, ctx->num_sms, false, s));
+		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, true, ls, ctx->num_sms, false, s));
 	} else if (ctx->mode == BBT_MODE_BESTHIT) {
 		ScoreArgs sa;
 		sa.scores[0] = sa.scores[1] = nullptr;

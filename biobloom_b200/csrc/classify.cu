@@ -221,8 +221,8 @@ __device__ __noinline__ void classify_long(const ClassifyArgs &a, uint64_t r, un
 			__syncwarp();
 		}
 		const int d = a.packed
-				? lane_long_item<MODE, false, COUNT, true>(a, nullptr, F, f, tab, r, words, lane, acc)
-				: lane_long_item<MODE, false, COUNT, false>(a, nullptr, F, f, tab, r, words, lane,
+				? lane_long_item<MODE, kLaneHits, COUNT, true>(a, nullptr, F, f, tab, r, words, lane, acc)
+				: lane_long_item<MODE, kLaneHits, COUNT, false>(a, nullptr, F, f, tab, r, words, lane,
 						acc);
 		if (d == EVAL_ACCEPT && lane == (int)(f >> 6))
 			myword |= 1ull << (f & 63);

@@ -103,9 +103,10 @@ __global__ void lane_long_kernel(ClassifyArgs a, uint32_t max_bases, uint32_t *l
 /* Items of chunk c, reads [32c, 32c + 32), into the warp's queue: those long
  * enough for a frame and not on the long list; the result of a read without
  * frames is written here.  Returns their number. */
-template <int MODE, bool SCORE, bool PACKED>
+template <int MODE, int WHAT, bool PACKED>
 __device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, uint64_t c, int lane)
 {
+	constexpr bool SCORE = WHAT != kLaneHits, HITS = WHAT != kLaneScores;
 	const ClassifyArgs &a = g.a;
 	const uint64_t r = c * 32 + lane;
 	const bool in = r < a.n * a.mates;
@@ -124,9 +125,9 @@ __device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, 
 			score_init(st);
 			g.sa.scores[mate][i * a.nf + g.f] = MODE == SCORE_BINOMIAL
 					? binomial_score(l, g.F.k, 0, 0.0, lane) : score_value<MODE>(st, l, g.F.k, 0.0, lane);
-		} else if (a.nf == 1) {
-			a.hits[mate][i] = 0;
 		}
+		if (HITS && a.nf == 1)
+			a.hits[mate][i] = 0;
 	}
 	const bool mine = in && l >= g.F.k && l <= g.max_bases;
 	const unsigned m = __ballot_sync(kFull, mine);
@@ -136,7 +137,7 @@ __device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, 
 		w.base[q] = b;
 		w.read[q] = (uint32_t)r;
 		w.len[q] = (uint32_t)l;
-		if (!SCORE) {
+		if (HITS) {
 			int32_t t, at;
 			double ht;
 			lane_thresholds<MODE>(t, at, ht, a.score, a.one_minus, a.min_len,
@@ -190,10 +191,11 @@ __device__ __forceinline__ void lane_count(const ClassifyArgs &a, unsigned long 
 	}
 }
 
-template <int MODE, bool SCORE, bool COUNT, bool PACKED>
+template <int MODE, int WHAT, bool COUNT, bool PACKED>
 __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 		const __grid_constant__ LaneArgs g)
 {
+	constexpr bool SCORE = WHAT != kLaneHits, HITS = WHAT != kLaneScores;
 	__shared__ LaneWarp<MODE> warps[kLaneWarps];
 	__shared__ LaneTables tab;
 	__shared__ double terms[MODE == SCORE_HARMONIC ? kHarmTerms : 1];
@@ -219,9 +221,9 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			if (it >= nlong)
 				break;
 			const uint32_t r = g.list[it];
-			const int d = lane_long_item<MODE, SCORE, COUNT, PACKED>(a, &g.sa, g.F, g.f, tab, r,
+			const int d = lane_long_item<MODE, WHAT, COUNT, PACKED>(a, &g.sa, g.F, g.f, tab, r,
 					&w.nib[0][0], lane, COUNT ? acc : nullptr);
-			if (!SCORE && lane == 0)
+			if (HITS && lane == 0)
 				lane_write(g, r, d);
 			__syncwarp();
 		}
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 	bool more = true;
 	int qi = 0, qn = 0;         /* queue: next item, items */
 	bool active = false;
+	bool open = false;          /* both: the decision has not fallen */
 	uint32_t pos = 0, run = 0;
 	uint64_t F = 0, R = 0;
 	LaneEval<MODE> ev;
@@ -251,7 +254,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 					more = c < g.chunks;
 					if (!more)
 						break;
-					qn = lane_queue<MODE, SCORE, PACKED>(g, w, c, lane);
+					qn = lane_queue<MODE, WHAT, PACKED>(g, w, c, lane);
 					qi = 0;
 					if (!qn)
 						continue;
@@ -266,10 +269,12 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 #pragma unroll
 					for (int j = 0; j < 4; ++j)
 						w.nib[j][lane] = 0;
-					if (SCORE) {
+					if (SCORE)
 						sc.start();
-					} else {
+					if (HITS) {
 						ev.start();
+						if (WHAT == kLaneBoth)
+							open = true;
 						w.my_thres[lane] = w.thres[q];
 						w.my_anti_thres[lane] = w.anti_thres[q];
 						if (MODE == SCORE_HARMONIC)
@@ -305,7 +310,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			const uint32_t hi = q8 == 1u ? nib : w.nib[(at - q8 + 1u) & 3u][lane];
 			w.nib[at & 3u][lane] = nib;
 			pairs = nib | (__funnelshift_r(lo, hi, 4u * (8u * q8 - g.F.k)) << 2);
-			if (!SCORE) {
+			if (HITS) {
 				ev.thres = w.my_thres[lane];
 				ev.anti_thres = w.my_anti_thres[lane];
 				if (MODE == SCORE_HARMONIC)
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 #pragma unroll 1
 		for (int s = 0; s < 8 / kLaneSub; ++s, p0 += kLaneSub) {
 			constexpr uint32_t kMask = (1u << kLaneSub) - 1u;
-			const uint32_t Vs = decided ? 0u : V & kMask;
+			const uint32_t Vs = !SCORE && decided ? 0u : V & kMask;
 			V >>= kLaneSub;
 			uint64_t canon[kLaneSub];
 #pragma unroll
@@ -341,10 +346,9 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			}
 			uint32_t cost[COUNT ? kLaneSub : 1];
 			live = lane_levels<COUNT, kLaneSub>(g.F, canon, live, pol, cost);
-			if (SCORE) {
-				if (Vs)
-					sc.template step<kLaneSub>(Vs, live, p0, k, (int32_t)a.streak_thr, terms);
-			} else if (Vs) {
+			if (SCORE && Vs)
+				sc.template step<kLaneSub>(Vs, live, p0, k, (int32_t)a.streak_thr, terms);
+			if (HITS && Vs && (WHAT != kLaneBoth || open)) {
 				uint32_t vis = 0;
 				decided = ev.template step<kLaneSub>(Vs, live, p0, k, (int32_t)a.streak_thr,
 						terms, COUNT ? &vis : nullptr);
@@ -356,7 +360,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			}
 		}
 		pos += 8u;
-		const bool done = active && (decided != EVAL_OPEN || pos >= w.my_len[lane]);
+		const bool done = active && ((!SCORE && decided != EVAL_OPEN) || pos >= w.my_len[lane]);
 		if (SCORE) {
 			const uint32_t read = w.my_read[lane], len = w.my_len[lane];
 			const uint32_t mate = read >= a.n ? 1u : 0u;
@@ -376,19 +380,22 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 			} else if (done) {
 				*out = score_value<MODE>(st, len, g.F.k, 0.0, lane);
 			}
-		} else if (done) {
+		}
+		/* both: the decision when it falls, or with the score */
+		if (HITS && (WHAT == kLaneBoth ? active && open && (decided != EVAL_OPEN || done) : done)) {
 			lane_write(g, w.my_read[lane], decided);
+			open = false;
 		}
 		active = active && !done;
 	}
 	lane_count<COUNT>(a, acc, lane);
 }
 
-template <int MODE, bool SCORE, bool COUNT>
+template <int MODE, int WHAT, bool COUNT>
 cudaError_t launch_mode(const LaneArgs &g, int num_sms, cudaStream_t s)
 {
-	auto kern = g.a.packed ? lane_kernel<MODE, SCORE, COUNT, true>
-	                       : lane_kernel<MODE, SCORE, COUNT, false>;
+	auto kern = g.a.packed ? lane_kernel<MODE, WHAT, COUNT, true>
+	                       : lane_kernel<MODE, WHAT, COUNT, false>;
 	int per_sm = 0;
 	cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kLaneWarps * 32, 0);
 	/* no more shared memory carved out than the blocks use: the rest is L1, which
@@ -409,14 +416,14 @@ cudaError_t launch_mode(const LaneArgs &g, int num_sms, cudaStream_t s)
 	return cudaGetLastError();
 }
 
-template <bool SCORE, bool COUNT>
+template <int WHAT, bool COUNT>
 cudaError_t launch_lane_as(const LaneArgs &g, int num_sms, cudaStream_t s)
 {
 	switch (g.a.scoring) {
-	case BBT_SCORE_LENGTH: return launch_mode<SCORE_LENGTH, SCORE, COUNT>(g, num_sms, s);
-	case BBT_SCORE_HARMONIC: return launch_mode<SCORE_HARMONIC, SCORE, COUNT>(g, num_sms, s);
-	case BBT_SCORE_BINOMIAL: return launch_mode<SCORE_BINOMIAL, SCORE, COUNT>(g, num_sms, s);
-	default: return launch_mode<SCORE_SIMPLE, SCORE, COUNT>(g, num_sms, s);
+	case BBT_SCORE_LENGTH: return launch_mode<SCORE_LENGTH, WHAT, COUNT>(g, num_sms, s);
+	case BBT_SCORE_HARMONIC: return launch_mode<SCORE_HARMONIC, WHAT, COUNT>(g, num_sms, s);
+	case BBT_SCORE_BINOMIAL: return launch_mode<SCORE_BINOMIAL, WHAT, COUNT>(g, num_sms, s);
+	default: return launch_mode<SCORE_SIMPLE, WHAT, COUNT>(g, num_sms, s);
 	}
 }
 
@@ -452,7 +459,7 @@ bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads)
 }
 
 cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreArgs *sa,
-		const LaneScratch &ls, int num_sms, bool count, cudaStream_t s)
+		bool hits, const LaneScratch &ls, int num_sms, bool count, cudaStream_t s)
 {
 	const uint64_t total = a.n * a.mates;
 	if (total == 0)
@@ -475,9 +482,10 @@ cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreA
 	g.ctr = ls.ctr + 1;
 	for (g.f = 0; g.f < a.nf; ++g.f, g.ctr += 2) {
 		g.F = lane_filter(hf[g.f]);
-		e = sa ? launch_lane_as<true, false>(g, num_sms, s)
-		  : count ? launch_lane_as<false, true>(g, num_sms, s)
-		          : launch_lane_as<false, false>(g, num_sms, s);
+		e = sa ? (hits ? launch_lane_as<kLaneBoth, false>(g, num_sms, s)
+		               : launch_lane_as<kLaneScores, false>(g, num_sms, s))
+		  : count ? launch_lane_as<kLaneHits, true>(g, num_sms, s)
+		          : launch_lane_as<kLaneHits, false>(g, num_sms, s);
 		if (e != cudaSuccess)
 			return e;
 	}

@@ -31,10 +31,10 @@ inline size_t lane_counters(uint32_t nf)
 }
 
 /* Hits of a batch (sa NULL), or the scores of every (read, filter) into
- * sa->scores.  With two or more filters the hit words are ORed into and must be
+ * sa->scores, and with `hits` both in one walk (count: hits alone).  With two or more filters the hit words are ORed into and must be
  * zeroed before. */
 cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreArgs *sa,
-		const LaneScratch &ls, int num_sms, bool count, cudaStream_t s);
+		bool hits, const LaneScratch &ls, int num_sms, bool count, cudaStream_t s);
 
 } // namespace bbt
 

@@ -46,6 +46,10 @@ __host__ __device__ inline LaneFilter lane_filter(const FilterDev &F)
 
 #if defined(__CUDACC__)
 
+/* What a walk is for: decisions, scores, or both (the frames that a decision
+ * visits are the first of those that a score does, with the same skip windows). */
+enum { kLaneHits = 0, kLaneScores = 1, kLaneBoth = 2 };
+
 /* Rolling tables of the filter's k, by outgoing code << 2 | incoming code, and
  * the hashes of k bases of code 0. */
 struct LaneTables {
@@ -295,11 +299,12 @@ __device__ __forceinline__ bool lane_long_plain(SimpleState &st, uint32_t V, uin
  * latency of h dependent probes; their hit bits then go through the warp's
  * chunk machine 32 at a time.  A window is no longer than the frames that the
  * earliest decision needs.  wmem: 16 words. */
-template <int MODE, bool SCORE, bool COUNT, bool PACKED>
+template <int MODE, int WHAT, bool COUNT, bool PACKED>
 __device__ __noinline__ int lane_long_item(const ClassifyArgs &a, const ScoreArgs *sa,
 		const LaneFilter f, uint32_t fi, const LaneTables &tab, uint64_t r, uint32_t *wmem,
 		int lane, unsigned long long *acc)
 {
+	constexpr bool SCORE = WHAT != kLaneHits, HITS = WHAT != kLaneScores;
 	const int k = (int)f.k;
 	const uint64_t pol = lane_policy(f.keep != 0);
 	const uint32_t mate = r >= a.n ? 1u : 0u;
@@ -314,6 +319,8 @@ __device__ __noinline__ int lane_long_item(const ClassifyArgs &a, const ScoreArg
 	ScoreState sc;
 	if (SCORE)
 		score_init(sc);
+	if (!HITS)
+		;
 	else if (MODE == SCORE_HARMONIC)
 		harmonic_init(qs, a.score, a.one_minus, frames);
 	else if (MODE == SCORE_BINOMIAL)
@@ -324,7 +331,7 @@ __device__ __noinline__ int lane_long_item(const ClassifyArgs &a, const ScoreArg
 		simple_init(st, a.score, a.one_minus, frames);
 	int decided = EVAL_OPEN;
 	int wn;
-	for (uint64_t w0 = 0; w0 < frames && !decided; w0 += wn) {
+	for (uint64_t w0 = 0; w0 < frames && (SCORE || !decided); w0 += wn) {
 		wn = 256;
 		if (!SCORE) {
 			if (MODE == SCORE_LENGTH)
@@ -358,14 +365,16 @@ __device__ __noinline__ int lane_long_item(const ClassifyArgs &a, const ScoreArg
 				lane_long_plain(st, V, live, wn, (int)a.streak_thr, lane))
 			continue;
 		uint32_t seen = 0; /* COUNT: this lane's frames that the algorithm probes */
-		for (int c = 0; c < wn && !decided; c += 32) {
+		for (int c = 0; c < wn && (SCORE || !decided); c += 32) {
 			const uint32_t Vc = vw[c >> 5], Hc = hw[c >> 5];
 			const int nf = min(32, wn - c);
 			const int64_t b = (int64_t)w0 + c;
 			uint32_t alg = 0;
 			if (SCORE)
 				score_chunk(sc, Vc, Hc, b, nf, k, a.streak_thr, MODE);
-			else if (MODE == SCORE_LENGTH)
+			if (!HITS || decided)
+				continue;
+			if (MODE == SCORE_LENGTH)
 				decided = length_chunk(ls, Vc, Hc, b, nf, COUNT ? &alg : nullptr);
 			else if (MODE == SCORE_HARMONIC)
 				decided = seq_chunk(qs, Vc, Hc, b, nf, k, a.streak_thr, COUNT ? &alg : nullptr);

@@ -21,11 +21,11 @@
  * over all k-mers (first numbers, new k-mers) with the slice's bits packed
  * between them.  Sequences that fit one chunk are copied to the device once.
  *
- * 20 Mbp (a 13.7 MB filter): 24 -> 15 ms, of which the kernels 3.1 -> 2.8.  The first-number pass is the larger
- * part of the kernels (2.2 ms: 60 M atomics over 440 MB, at the rate that
- * isolated read-modify-writes of HBM reach, 27 G/s of it); an insertion pass of
- * its own (0.35 ms), a copy of the sequences per pass and the redundancy
- * integral on one thread (most of the time) are gone.
+ * 20 Mbp (a 13.7 MB filter): 24 -> 15 ms, of which the kernels 3.1 -> 2.8.  The
+ * first-number pass is the larger part of these (2.2 ms: 60 M atomics over 440
+ * MB, 27 G/s, what isolated read-modify-writes of HBM reach); an insertion pass
+ * of its own (0.35 ms), a copy of the sequences per pass and the redundancy
+ * integral on one thread are gone.
  */
 #include <cuda_runtime.h>
 

@@ -335,12 +335,13 @@ __global__ void __launch_bounds__(kScanThreads, kScanBlocks) mibf_scan_kernel(
 		if (r0 + lane <= r1) {
 			o1 = g.off[r0 + lane];
 			o2 = g.seq2 ? g.off2[r0 + lane] : 0;
-			if (r0 + lane < r1) {
-				scan_prefetch(mate_bases(g, 0, o1));
-				if (g.seq2)
-					scan_prefetch(mate_bases(g, 1, o2));
-			}
 		}
+		const bool has1 = __shfl_down_sync(kFull, o1, 1) > o1;
+		const bool has2 = __shfl_down_sync(kFull, o2, 1) > o2;
+		if (r0 + lane < r1 && has1)
+			scan_prefetch(mate_bases(g, 0, o1));
+		if (r0 + lane < r1 && has2)
+			scan_prefetch(mate_bases(g, 1, o2));
 		for (uint64_t r = r0; r < r1; ++r) {
 			const int j = (int)(r - r0);
 			const uint64_t b1 = __shfl_sync(kFull, o1, j), b2 = __shfl_sync(kFull, o2, j);

@@ -53,8 +53,11 @@ extern "C" {
 /* ---- kernel paths ---- */
 #define BBT_PATH_AUTO 0        /* persistent work-stealing path, tuned */
 #define BBT_PATH_PLAIN 1       /* one warp per read, one launch per batch */
-#define BBT_PATH_PERSISTENT 2  /* persistent work-stealing kernel, read-major */
-#define BBT_PATH_FILTER_MAJOR 3 /* persistent, (filter, read) items in filter order */
+#define BBT_PATH_PERSISTENT 2  /* persistent work-stealing kernels: a read per lane from
+                                  20,000 reads on (28,000 over filters in HBM), a read per
+                                  warp below */
+#define BBT_PATH_FILTER_MAJOR 3 /* one filter after another: a read per lane as above, below
+                                  that hashes stored once and (filter, read) items */
 #define BBT_PATH_BUCKETED 4    /* probes sorted by filter address (filters far above L2) */
 
 typedef struct bbt_ctx bbt_ctx;
@@ -358,7 +361,8 @@ typedef struct {
 } bbt_tune;
 int bbt_autotune(bbt_ctx *ctx, const bbt_batch *sample, bbt_tune *out);
 
-/* Steps of the persistent path.  Each step of a warp probes up to 32 frames
+/* Steps of the persistent path's warp kernel (the one with a read per lane takes
+ * the batches above where this is BBT_STEPS_DECISION).  Each step of a warp probes up to 32 frames
  * of a read, one per lane, or up to 64 with two frames per lane (WIDE: twice
  * the filter reads in flight, for filters in HBM where the kernel waits on
  * them).  With SIMPLE and BINOMIAL scoring, DECISION steps are sized to the

@@ -271,3 +271,29 @@ def test_long_reads_of_small_batches(tmp_path, ks, h, scoring, score, streak, pa
                 alg += a
                 assert np.array_equal(t.cpu().numpy().view(np.uint64), w)
         assert bbc.last_stats()["probes_algorithmic"] == alg
+
+
+@pytest.mark.parametrize("ks,scoring,score,paired", [([25], ol.SIMPLE, 0.15, False),
+                                                     ([25, 25], ol.SIMPLE, 0.6, True),
+                                                     ([25, 21], ol.HARMONIC, 0.15, False),
+                                                     ([18, 25], ol.LENGTH, 40, True),
+                                                     ([25], ol.BINOMIAL, 100, False)])
+def test_hits_beside_scores(tmp_path, ks, scoring, score, paired):
+    """SCORES mode takes hits and scores from one walk: the hits are those of a
+    call without scores."""
+    import torch
+    from biobloom_b200 import MODE_SCORES
+    rng = np.random.default_rng(120 + scoring + len(ks))
+    genomes, filters, paths = _filters(tmp_path, rng, ks, 3)
+    n = 20100 // (2 if paired else 1) + 3
+    mates = [_reads(rng, genomes, n, ks[0]) for _ in range(2 if paired else 1)]
+    thr = 10.0 ** (-score / 10.0) if scoring == ol.BINOMIAL else score
+    dev = [t for m in mates for t in _device(m, 1)]
+    with _open(paths, scoring, score, 3) as bbc:
+        bbc.set_mode(MODE_SCORES)
+        sc = [torch.full((n, len(ks)), -7.0, dtype=torch.float64, device="cuda") for _ in mates]
+        got = bbc.classify_device(*dev, scores=sc[0], scores2=sc[1] if paired else None)
+        torch.cuda.synchronize()
+    for m, t in zip(mates, got[:2]):
+        want, _ = ol.classify(*ol.pack_reads(m), filters, thr, 3, scoring=scoring)
+        assert np.array_equal(t.cpu().numpy().view(np.uint64), want)
