@@ -1211,7 +1211,8 @@ static bool lane_wanted(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t tot
 {
 	const bool path = lc.path == BBT_PATH_FILTER_MAJOR ||
 			(lc.path == BBT_PATH_PERSISTENT && lc.steps == BBT_STEPS_DECISION);
-	return path && lane_pays(ctx->hf.data(), ctx->nf, total) &&
+	const bool scores = ctx->mode == BBT_MODE_BESTHIT || ctx->mode == BBT_MODE_SCORES;
+	return path && lane_pays(ctx->hf.data(), ctx->nf, total, scores) &&
 			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total);
 }
 

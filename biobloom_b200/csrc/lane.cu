@@ -448,14 +448,29 @@ static bool lane_in_l2(const FilterDev *hf, uint32_t nf)
 	return false;
 }
 
-/* A lane's read takes its time (80 us for 150 bases over a filter in L2, 115-138 us
- * over one in HBM, whatever the batch's size); the warp kernels' time grows with
- * the batch and reaches that at about these sizes (reads of 150 bases: 78 us per
- * 20k reads, 68 per 16k, 106 per 32k in L2; 122 us per 24k, 151 per 32k in HBM; ten filters
- * of 68 MB: 743 us per 16k reads and 1232 per 32k, against 850). */
-bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads)
+/* A lane's read takes its time (82 us for 150 bases over a filter in L2, 115-138 us
+ * over one in HBM, the same for any batch of up to 37,888 reads); the other kernels'
+ * time grows with the batch and reaches that at about 20k reads in L2 (82 us) and 28k
+ * in HBM (122 us per 24k, 151 per 32k).  So it does with a few filters (four: 267
+ * against 270 us at 20k) and with many that do not fit L2 together (ten of 68 MB: 927
+ * against 836 at 20k).  Many that do fit are another matter: the filter-major passes
+ * hash a read once for all of them and find them all in L2, the lane kernel pays a
+ * launch's latency for each.  Ten of 3.4 MB meet at 50k reads (852 against 867 us;
+ * 20k: 433 against 637), thirty at 60k (2584 against 2575; 20k: 954 against 1865).
+ * Scores are walked per filter either way: ten meet at 20k (621 against 634), thirty
+ * at 28k (1852 against 1857; 20k: 1410 against 1843). */
+bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads, bool scores)
 {
-	return total_reads >= (lane_in_l2(hf, nf) ? 20000u : 28000u);
+	if (!lane_in_l2(hf, nf))
+		return total_reads >= 28000;
+	uint64_t bytes = 0;
+	for (uint32_t i = 0; i < nf; ++i)
+		bytes += hf[i].m / 8;
+	if (nf <= 4 || bytes > kLaneKeepBytes)
+		return total_reads >= 20000;
+	if (scores)
+		return total_reads >= (nf <= 10 ? 20000u : 28000u);
+	return total_reads >= std::min<uint64_t>(60000, 5000ull * nf);
 }
 
 cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreArgs *sa,

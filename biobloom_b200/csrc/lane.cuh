@@ -21,7 +21,7 @@ struct LaneScratch {
 /* Whether the lane kernel takes these filters and options, and whether it is the
  * faster one for a batch of so many reads. */
 bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64_t total_reads);
-bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads);
+bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads, bool scores);
 
 /* Counters of a launch (which is a kernel per filter, after one that lists long
  * reads). */

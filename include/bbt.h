@@ -54,8 +54,9 @@ extern "C" {
 #define BBT_PATH_AUTO 0        /* persistent work-stealing path, tuned */
 #define BBT_PATH_PLAIN 1       /* one warp per read, one launch per batch */
 #define BBT_PATH_PERSISTENT 2  /* persistent work-stealing kernels: a read per lane from
-                                  20,000 reads on (28,000 over filters in HBM), a read per
-                                  warp below */
+                                  20,000 reads on (28,000 over filters in HBM, up to 60,000
+                                  over many filters that fit L2 together), a read per warp
+                                  below */
 #define BBT_PATH_FILTER_MAJOR 3 /* one filter after another: a read per lane as above, below
                                   that hashes stored once and (filter, read) items */
 #define BBT_PATH_BUCKETED 4    /* probes sorted by filter address (filters far above L2) */

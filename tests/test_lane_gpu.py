@@ -297,3 +297,34 @@ def test_hits_beside_scores(tmp_path, ks, scoring, score, paired):
     for m, t in zip(mates, got[:2]):
         want, _ = ol.classify(*ol.pack_reads(m), filters, thr, 3, scoring=scoring)
         assert np.array_equal(t.cpu().numpy().view(np.uint64), want)
+
+
+@pytest.mark.parametrize("nf,n,mode,lane", [
+    (4, 19999, "std", False), (4, 20000, "std", True), (5, 24999, "std", False),
+    (5, 25000, "std", True), (5, 20000, "best", True), (13, 59999, "std", False),
+    (13, 60000, "std", True), (11, 27999, "best", False), (11, 28000, "best", True)])
+def test_many_small_filters_choose_by_reads(tmp_path, nf, n, mode, lane):
+    """Either side of the sizes from which several filters in L2 take the lane kernel
+    (one launch a filter, against one for all)."""
+    import torch
+    from biobloom_b200 import MODE_BESTHIT, BioBloomClassifier
+    from biobloom_b200 import _lib as L
+    rng = np.random.default_rng(nf * 100000 + n)
+    genomes, filters, paths = _filters(tmp_path, rng, [25] * nf, 3, glen=3000)
+    reads = []
+    for size in rng.integers(0, 60, n):
+        g = genomes[int(rng.integers(0, nf))]
+        st = int(rng.integers(0, len(g) - size))
+        reads.append(g[st:st + size].tobytes())
+    seq, off = ol.pack_reads(reads)
+    if mode == "best":
+        want, _ = ol.best_hit(ol.classify_scores(seq, off, filters, ol.SIMPLE, 3))
+    else:
+        want, _ = ol.classify(seq, off, filters, 0.15, 3)
+    with BioBloomClassifier(paths, 0.15, streak_threshold=3, path=L.PATH_PERSISTENT) as bbc:
+        if mode == "best":
+            bbc.set_mode(MODE_BESTHIT)
+        got = bbc.classify_device(*_device(reads, 0))
+        torch.cuda.synchronize()
+        assert np.array_equal(got[0].cpu().numpy().view(np.uint64), want)
+        assert (bbc.last_stats()["kernels"] > nf) == lane
