@@ -150,6 +150,15 @@ static void flush_slot(Slot &s)
 	s.pending.clear();
 }
 
+/* The counters of a scratch, which every call may use; its buffers come as they
+ * are needed. */
+static cudaError_t scratch_counters(const bbt_ctx *ctx, BfScratch &sc)
+{
+	cudaError_t e = cudaMalloc(&sc.work, sizeof(unsigned long long));
+	return e != cudaSuccess ? e : cudaMalloc(&sc.order_cnt,
+			order_counters(ctx->nf) * sizeof(unsigned long long));
+}
+
 extern "C" int bbt_close(bbt_ctx *ctx)
 {
 	if (!ctx)
@@ -168,18 +177,13 @@ extern "C" int bbt_close(bbt_ctx *ctx)
 		cudaFree(w);
 	cudaFree(ctx->d_filters);
 	cudaFree(ctx->d_fpr);
-	cudaFree(ctx->d_tmp_scores[0]);
-	cudaFree(ctx->d_tmp_scores[1]);
 	cudaFree(ctx->d_dust[0]);
 	cudaFree(ctx->d_dust[1]);
 	cudaFree(ctx->d_dust_redo);
 	cudaFree(ctx->d_dust_cnt);
 	cudaFree(ctx->d_dust_scratch);
 	cudaFree(ctx->d_counts);
-	cudaFree(ctx->d_work);
-	cudaFree(ctx->d_order);
-	cudaFree(ctx->d_order_cnt);
-	cudaFree(ctx->d_lane_list);
+	bf_scratch_free(ctx->sc);
 	cudaFree(ctx->d_bthres);
 	cudaFree(ctx->d_lenset);
 	cudaFree(ctx->d_stat);
@@ -521,9 +525,7 @@ extern "C" int bbt_open(const char *const *bf_paths, int n_filters, const bbt_pa
 			cudaMemcpyHostToDevice));
 	OPEN_TRY(cudaMalloc(&ctx->d_counts, sizeof(unsigned long long) * (2 * (ctx->nf + 2) + 2)));
 	OPEN_TRY(cudaMemset(ctx->d_counts, 0, sizeof(unsigned long long) * (2 * (ctx->nf + 2) + 2)));
-	OPEN_TRY(cudaMalloc(&ctx->d_work, sizeof(unsigned long long)));
-	OPEN_TRY(cudaMalloc(&ctx->d_order_cnt, order_counters(ctx->nf) *
-			sizeof(unsigned long long)));
+	OPEN_TRY(scratch_counters(ctx, ctx->sc));
 	OPEN_TRY(cudaMalloc(&ctx->d_stat, 3 * sizeof(unsigned long long)));
 	OPEN_TRY(cudaMemset(ctx->d_stat, 0, 3 * sizeof(unsigned long long)));
 	ctx->cap_reads = ctx->p.max_batch_reads ? ctx->p.max_batch_reads : (1ull << 20);
@@ -732,7 +734,7 @@ static ClassifyArgs base_args(const bbt_ctx *ctx)
 	a.kmax = ctx->kmax;
 	a.bthres = ctx->d_bthres;
 	a.bthres_rows = ctx->bt_rows;
-	a.work = ctx->d_work;
+	a.work = ctx->sc.work;
 	a.lane_long = ctx->lc.steps == BBT_STEPS_DECISION &&
 			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, 0);
 	if (ctx->lc.count) {
@@ -755,6 +757,25 @@ static int grow(bbt_ctx *ctx, T **buf, uint64_t &cap, uint64_t n)
 	CUDA_TRY(ctx, cudaMalloc(buf, std::max<uint64_t>(n, 1) * sizeof(T)));
 	cap = n;
 	return BBT_OK;
+}
+
+/* grow for scratch that the call can do without: false, and no error left, when
+ * there is no room for it. */
+template <typename T>
+static bool grow_if_room(T **buf, uint64_t &cap, uint64_t n)
+{
+	if (n <= cap)
+		return true;
+	cudaFree(*buf);
+	*buf = nullptr;
+	cap = 0;
+	if (cudaMalloc(buf, n * sizeof(T)) != cudaSuccess) {
+		cudaGetLastError();
+		*buf = nullptr;
+		return false;
+	}
+	cap = n;
+	return true;
 }
 
 /* Two-pass filter-major classification of one batch (all filters share k):
@@ -822,7 +843,7 @@ static int run_two_pass(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s,
 		p.k = k;
 		p.h0 = ctx->d_tp_h0;
 		p.vmask = ctx->d_tp_vmask;
-		p.work = ctx->d_work;
+		p.work = ctx->sc.work;
 		CUDA_TRY(ctx, two_pass_sub_batch(a, p, ctx->lc, s, sa, classify));
 	}
 	return BBT_OK;
@@ -1107,7 +1128,7 @@ static int run_bucketed(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s)
 			b.res = ctx->d_bk_res;
 			b.btot = ctx->d_bk_btot;
 			b.issued = a.probes;
-			b.next = ctx->d_work;
+			b.next = ctx->sc.work;
 			for (const auto &ph : phases) {
 				b.ph_lo = ph.first;
 				b.ph_hi = ph.second;
@@ -1143,7 +1164,7 @@ static int run_bucketed(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s)
 		one.order = nullptr;
 		LaunchConfig lc = ctx->lc;
 		lc.path = BBT_PATH_PERSISTENT;
-		CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long), s));
+		CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.work, 0, sizeof(unsigned long long), s));
 		CUDA_TRY(ctx, launch_classify(one, lc, s));
 		ctx->last.kernels += 1;
 	}
@@ -1216,11 +1237,20 @@ static bool lane_wanted(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t tot
 			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total);
 }
 
+/* BESTHIT by the lane kernel goes through stored scores: outside the
+ * filter-major path, whose batches always stored them, only while they stay
+ * within 1 GB. */
+static bool lane_stores_scores(const bbt_ctx *ctx, uint64_t n, uint32_t mates)
+{
+	return (ctx->lc.path == BBT_PATH_FILTER_MAJOR && ctx->same_k) ||
+			n * ctx->nf * mates <= (128ull << 20);
+}
+
 /* The lane kernel over a batch: hits (classify) and / or scores (sa). */
 static int run_lane(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreArgs *sa,
 		bool classify)
 {
-	const LaneScratch ls = {ctx->d_lane_list, ctx->d_order_cnt};
+	const LaneScratch ls = {ctx->sc.lane_list, ctx->sc.order_cnt};
 	const bool count = ctx->lc.count != 0;
 	const bool both = classify && sa && !count; /* one walk for hits and scores */
 	if (classify) {
@@ -1261,19 +1291,17 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	const bool two_pass = ctx->lc.path == BBT_PATH_FILTER_MAJOR && ctx->same_k;
 	const bool best_only = ctx->mode == BBT_MODE_BESTHIT && !want_scores;
 	bool lane = lane_wanted(ctx, ctx->lc, a.n * a.mates);
-	/* BESTHIT through stored scores: outside the filter-major path, whose
-	 * batches always stored them, only while they stay within 1 GB */
-	if (lane && best_only && !two_pass && a.n * ctx->nf * a.mates > (128ull << 20))
+	if (lane && best_only && !lane_stores_scores(ctx, a.n, a.mates))
 		lane = false;
 	/* scores of one mate only: the kernels that test each array */
 	if (lane && want_scores && (!sa.scores[0] || (a.mates == 2 && !sa.scores[1])))
 		lane = false;
-	/* no allocation while a graph is captured */
-	if (lane && ctx->capturing && (a.n * a.mates > ctx->lane_list_cap ||
-			(best_only && a.n * ctx->nf > ctx->tmp_scores_cap)))
+	/* no allocation while a graph is captured: with the scratch that it has */
+	if (lane && ctx->capturing && (a.n * a.mates > ctx->sc.lane_list_cap ||
+			(best_only && a.n * ctx->nf > ctx->sc.scores_cap)))
 		lane = false;
 	if (lane) {
-		int rc = grow(ctx, &ctx->d_lane_list, ctx->lane_list_cap, a.n * a.mates);
+		int rc = grow(ctx, &ctx->sc.lane_list, ctx->sc.lane_list_cap, a.n * a.mates);
 		if (rc)
 			return rc;
 	}
@@ -1284,17 +1312,17 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 		ScoreArgs ps = sa;
 		if (best_only) {
 			const uint64_t need = a.n * ctx->nf;
-			if (need > ctx->tmp_scores_cap) {
-				cudaFree(ctx->d_tmp_scores[0]);
-				cudaFree(ctx->d_tmp_scores[1]);
-				ctx->d_tmp_scores[0] = ctx->d_tmp_scores[1] = nullptr;
-				ctx->tmp_scores_cap = 0;
-				CUDA_TRY(ctx, cudaMalloc(&ctx->d_tmp_scores[0], need * sizeof(double)));
-				CUDA_TRY(ctx, cudaMalloc(&ctx->d_tmp_scores[1], need * sizeof(double)));
-				ctx->tmp_scores_cap = need;
+			if (need > ctx->sc.scores_cap) {
+				cudaFree(ctx->sc.scores[0]);
+				cudaFree(ctx->sc.scores[1]);
+				ctx->sc.scores[0] = ctx->sc.scores[1] = nullptr;
+				ctx->sc.scores_cap = 0;
+				CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[0], need * sizeof(double)));
+				CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[1], need * sizeof(double)));
+				ctx->sc.scores_cap = need;
 			}
-			ps.scores[0] = ctx->d_tmp_scores[0];
-			ps.scores[1] = a.mates == 2 ? ctx->d_tmp_scores[1] : nullptr;
+			ps.scores[0] = ctx->sc.scores[0];
+			ps.scores[1] = a.mates == 2 ? ctx->sc.scores[1] : nullptr;
 		}
 		const bool classify = ctx->mode != BBT_MODE_BESTHIT;
 		if (classify && !lane) {
@@ -1341,15 +1369,15 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 		if (lc.path == BBT_PATH_FILTER_MAJOR)
 			lc.path = BBT_PATH_PERSISTENT; /* filters of different k */
 		if (lc.path != BBT_PATH_PLAIN)
-			CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_work, 0, sizeof(unsigned long long), s));
+			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.work, 0, sizeof(unsigned long long), s));
 		if (lc.path != BBT_PATH_PLAIN && ctx->long_bases) {
-			int rc = grow(ctx, &ctx->d_order, ctx->order_cap, a.n * a.mates);
+			int rc = grow(ctx, &ctx->sc.order, ctx->sc.order_cap, a.n * a.mates);
 			if (rc)
 				return rc;
-			CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_order_cnt, 0, 2 * sizeof(unsigned long long), s));
-			CUDA_TRY(ctx, launch_long_first(a, ctx->long_bases, ctx->d_order, ctx->d_order_cnt,
+			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.order_cnt, 0, 2 * sizeof(unsigned long long), s));
+			CUDA_TRY(ctx, launch_long_first(a, ctx->long_bases, ctx->sc.order, ctx->sc.order_cnt,
 					ctx->num_sms, s));
-			a.order = ctx->d_order;
+			a.order = ctx->sc.order;
 			ctx->last.kernels += 1;
 		}
 		CUDA_TRY(ctx, launch_classify(a, lc, s));
@@ -2248,8 +2276,32 @@ struct bbt_graph {
 	cudaGraph_t graph = nullptr;
 	cudaGraphExec_t exec = nullptr;
 	cudaStream_t capture = nullptr;
+	BfScratch sc; /* what the captured launches use: a later call on the context may
+	                 replace the buffers of the context's own */
 	uint64_t reads = 0, launches = 0;
 };
+
+/* The scratch of a graph of launches of up to `reads` reads (pairs) each, before
+ * the capture, which cannot allocate.  Without room for what the lane kernel
+ * takes the capture holds the warp kernels. */
+static int graph_scratch(bbt_ctx *ctx, BfScratch &sc, uint64_t reads, uint32_t mates)
+{
+	CUDA_TRY(ctx, scratch_counters(ctx, sc));
+	if (ctx->long_bases && ctx->lc.path != BBT_PATH_PLAIN) {
+		int rc = grow(ctx, &sc.order, sc.order_cap, reads * mates);
+		if (rc)
+			return rc;
+	}
+	if (lane_wanted(ctx, ctx->lc, reads * mates) &&
+			grow_if_room(&sc.lane_list, sc.lane_list_cap, reads * mates) &&
+			ctx->mode == BBT_MODE_BESTHIT && lane_stores_scores(ctx, reads, mates)) {
+		uint64_t cap[2] = {0, 0};
+		for (uint32_t m = 0; m < mates; ++m)
+			grow_if_room(&sc.scores[m], cap[m], reads * ctx->nf);
+		sc.scores_cap = cap[0] && (mates == 1 || cap[1]) ? reads * ctx->nf : 0;
+	}
+	return BBT_OK;
+}
 
 extern "C" int bbt_graph_create(bbt_ctx *ctx, const bbt_batch *b, const bbt_result *r,
 		uint64_t reads_per_launch, bbt_graph **out)
@@ -2269,17 +2321,6 @@ extern "C" int bbt_graph_create(bbt_ctx *ctx, const bbt_batch *b, const bbt_resu
 	const uint64_t n = b->n_reads;
 	const uint64_t chunk = reads_per_launch ? std::min(reads_per_launch, std::max<uint64_t>(n, 1))
 	                                        : std::max<uint64_t>(n, 1);
-	/* buffers the launches grow must exist before capture */
-	if (ctx->long_bases && ctx->lc.path != BBT_PATH_PLAIN) {
-		int rc = grow(ctx, &ctx->d_order, ctx->order_cap, chunk * (b->seq2 ? 2 : 1));
-		if (rc)
-			return rc;
-	}
-	if (lane_wanted(ctx, ctx->lc, chunk * (b->seq2 ? 2 : 1))) {
-		int rc = grow(ctx, &ctx->d_lane_list, ctx->lane_list_cap, chunk * (b->seq2 ? 2 : 1));
-		if (rc)
-			return rc;
-	}
 	if (ctx->p.scoring == BBT_SCORE_BINOMIAL) { /* thresholds before capture */
 		std::vector<uint64_t> lens;
 		int rc = device_lengths(ctx, b, ctx->stream, lens);
@@ -2291,11 +2332,17 @@ extern "C" int bbt_graph_create(bbt_ctx *ctx, const bbt_batch *b, const bbt_resu
 	bbt_graph *g = new bbt_graph();
 	g->ctx = ctx;
 	g->reads = n;
+	int rc = graph_scratch(ctx, g->sc, chunk, b->seq2 ? 2 : 1);
+	if (rc) {
+		bbt_graph_destroy(g);
+		return rc;
+	}
+	std::swap(ctx->sc, g->sc);
 	ctx->capturing = true;
 	cudaError_t e = cudaStreamCreateWithFlags(&g->capture, cudaStreamNonBlocking);
 	if (e == cudaSuccess)
 		e = cudaStreamBeginCapture(g->capture, cudaStreamCaptureModeThreadLocal);
-	int rc = e == cudaSuccess ? BBT_OK : cuda_fail(ctx, e, "cudaStreamBeginCapture");
+	rc = e == cudaSuccess ? BBT_OK : cuda_fail(ctx, e, "cudaStreamBeginCapture");
 	for (uint64_t i = 0; rc == BBT_OK && i < n; i += chunk) {
 		bbt_batch sb = *b;
 		sb.n_reads = std::min(chunk, n - i);
@@ -2312,6 +2359,7 @@ extern "C" int bbt_graph_create(bbt_ctx *ctx, const bbt_batch *b, const bbt_resu
 	cudaGraph_t graph = nullptr;
 	e = cudaStreamEndCapture(g->capture, &graph);
 	ctx->capturing = false;
+	std::swap(ctx->sc, g->sc);
 	if (rc == BBT_OK && e != cudaSuccess)
 		rc = cuda_fail(ctx, e, "cudaStreamEndCapture");
 	g->graph = graph;
@@ -2358,6 +2406,7 @@ extern "C" int bbt_graph_destroy(bbt_graph *g)
 		cudaGraphDestroy(g->graph);
 	if (g->capture)
 		cudaStreamDestroy(g->capture);
+	bf_scratch_free(g->sc);
 	delete g;
 	return BBT_OK;
 }
@@ -2367,9 +2416,7 @@ extern "C" int bbt_graph_destroy(bbt_graph *g)
 int bbt::bf_scratch_init(bbt_ctx *ctx, BfScratch &sc, uint64_t max_reads)
 {
 	CUDA_TRY(ctx, cudaSetDevice(ctx->dev));
-	CUDA_TRY(ctx, cudaMalloc(&sc.work, sizeof(unsigned long long)));
-	CUDA_TRY(ctx, cudaMalloc(&sc.order_cnt, order_counters(ctx->nf) *
-			sizeof(unsigned long long)));
+	CUDA_TRY(ctx, scratch_counters(ctx, sc));
 	CUDA_TRY(ctx, cudaMalloc(&sc.order, std::max<uint64_t>(max_reads, 1) * 2 * sizeof(uint64_t)));
 	sc.order_cap = std::max<uint64_t>(max_reads, 1) * 2;
 	return BBT_OK;
@@ -2380,6 +2427,9 @@ void bbt::bf_scratch_free(BfScratch &sc)
 	cudaFree(sc.work);
 	cudaFree(sc.order_cnt);
 	cudaFree(sc.order);
+	cudaFree(sc.lane_list);
+	cudaFree(sc.scores[0]);
+	cudaFree(sc.scores[1]);
 	sc = BfScratch();
 }
 

@@ -48,6 +48,27 @@ struct Slot {
 
 void set_global_error(const std::string &msg);
 
+/* Counters of the read order (2) or of the lane kernel. */
+inline size_t order_counters(uint32_t nf)
+{
+	return std::max<size_t>(2, lane_counters(nf));
+}
+
+/* Device scratch of classification calls that run one after another.  The
+ * context's own calls share one, whose buffers grow with the batches; what may
+ * run beside them or outlive a buffer that they replace has its own: each
+ * stream of the serving engine, each captured graph. */
+struct BfScratch {
+	unsigned long long *work = nullptr;      /* persistent kernels' read counter */
+	unsigned long long *order_cnt = nullptr; /* order_counters(nf) words */
+	uint64_t *order = nullptr;               /* long-first read order */
+	uint64_t order_cap = 0;
+	uint32_t *lane_list = nullptr;           /* lane kernel (lane.cu): the batch's long reads */
+	uint64_t lane_list_cap = 0;
+	double *scores[2] = {nullptr, nullptr};  /* BESTHIT scores nobody asked for */
+	uint64_t scores_cap = 0;                 /* elements per mate array */
+};
+
 } // namespace bbt
 
 struct bbt_ctx {
@@ -64,7 +85,7 @@ struct bbt_ctx {
 	bbt::FilterDev *d_filters = nullptr;
 	uint32_t nf = 0, words = 0, kmax = 0;
 	unsigned long long *d_counts = nullptr; /* 2*(nf+2)+2 summary counters */
-	unsigned long long *d_work = nullptr;   /* persistent-kernel read counter */
+	bbt::BfScratch sc;
 	unsigned long long *d_stat = nullptr;   /* probes, frames */
 	uint64_t reads_seen = 0;
 	bbt::Slot slot[2];
@@ -74,8 +95,6 @@ struct bbt_ctx {
 	/* filtering mode (BBT_MODE_*): ORDERED, BESTHIT and SCORES */
 	int mode = BBT_MODE_STD;
 	double *d_fpr = nullptr;         /* each filter's FPR on the device (BINOMIAL scores) */
-	double *d_tmp_scores[2] = {nullptr, nullptr}; /* BESTHIT scores nobody asked for */
-	uint64_t tmp_scores_cap = 0;                  /* elements per mate array */
 	/* -D: SDUST masking before classification (dust.cu) */
 	bool dust = false;
 	int dust_T = 20, dust_W = 64;
@@ -113,12 +132,6 @@ struct bbt_ctx {
 	bool to_stdout = false, inverse = false;
 	/* long-first read order of the persistent kernel (0 = index order) */
 	uint64_t long_bases = 0;
-	uint64_t *d_order = nullptr;
-	uint64_t order_cap = 0;
-	unsigned long long *d_order_cnt = nullptr; /* order_counters(nf) words */
-	/* lane kernel (lane.cu): the batch's long reads */
-	uint32_t *d_lane_list = nullptr;
-	uint64_t lane_list_cap = 0;
 	/* bucketed probe path (bucketed.cu): frame offsets of a batch's reads and
 	 * their host samples, per-read state, the batch's bases as 2-bit codes
 	 * (ASCII batches), validity / hit / requesting bits and canonical hashes
@@ -161,22 +174,9 @@ struct bbt_ctx {
 };
 
 namespace bbt {
-/* Counters of the read order (2) or of the lane kernel. */
-inline size_t order_counters(uint32_t nf)
-{
-	return std::max<size_t>(2, lane_counters(nf));
-}
 int fail(bbt_ctx *ctx, int code, const std::string &msg);
 
-/* Per-stream scratch for classification calls that run concurrently on
- * several streams of one context (the serving engine): each stream needs its
- * own work counter and read-order buffer. */
-struct BfScratch {
-	unsigned long long *work = nullptr;
-	unsigned long long *order_cnt = nullptr;
-	uint64_t *order = nullptr;
-	uint64_t order_cap = 0;
-};
+/* Scratch of one stream of the serving engine, for up to max_reads reads (pairs). */
 int bf_scratch_init(bbt_ctx *ctx, BfScratch &sc, uint64_t max_reads);
 /* BINOMIAL: allocate threshold rows for reads up to max_len bases up front
  * (the serving engine, so that the table never moves under running kernels),

@@ -383,7 +383,9 @@ int bbt_set_steps(bbt_ctx *ctx, int steps);
  * bbt_graph_launch: the launch sequence (work-counter resets, read order,
  * classification and summary kernels per launch) costs one graph launch.  The
  * graph is bound to the batch's and results' device pointers: refill those
- * buffers between launches.  Summary counters are updated at each launch.
+ * buffers between launches.  It holds what else its launches use: other calls
+ * on the context may come between them, of any size (BESTHIT graphs hold up to
+ * 1 GB for their scores).  Summary counters are updated at each launch.
  * Plain and persistent paths only (the filter-major path reads block sums on
  * the host).  Create it after a warm-up call with the same sizes.
  */
