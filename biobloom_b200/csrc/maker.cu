@@ -40,6 +40,7 @@
 #include "bbt_device.cuh"
 #include "ctx.hpp"
 #include "formats.hpp"
+#include "ordered_sum.hpp"
 
 namespace bbt {
 namespace {
@@ -140,21 +141,6 @@ __global__ void popcount_kernel(const uint32_t *w, uint64_t n, unsigned long lon
 		atomicAdd(&counts[1], c);
 }
 
-/* fn(lo, hi) over [0, n) in equal parts, one per thread (up to 8, for at least
- * 1024 elements each). */
-template <class Fn>
-void on_threads(uint64_t n, Fn fn)
-{
-	const uint64_t most = std::min<uint64_t>(8, std::max(1u, std::thread::hardware_concurrency()));
-	const uint64_t parts = std::max<uint64_t>(1, std::min(most, n / 1024));
-	std::vector<std::thread> th;
-	for (uint64_t p = 1; p < parts; ++p)
-		th.emplace_back(fn, n * p / parts, n * (p + 1) / parts);
-	fn(0, n / parts);
-	for (std::thread &t : th)
-		t.join();
-}
-
 /* BloomFilterInfo::calcRedunancyFPR (Common/BloomFilterInfo.cpp:289-297) is
  * sum_{i=1}^{n-1} approxFPR(size, i, h) / n; it is evaluated exactly up to
  * 2^20 terms and by Simpson's rule (a smooth, monotone integrand) above. */
@@ -165,32 +151,15 @@ double redundancy_fpr(uint64_t size, uint64_t n, unsigned h)
 	auto f = [&](double i) {
 		return std::pow(1.0 - std::exp(i * h * std::log1p(-1.0 / (double)size)), (double)h);
 	};
-	/* the terms on several threads, their sum in order: the same value on any
-	 * number of them */
-	double sum = 0;
-	if (n <= (1u << 20)) {
-		std::vector<double> t((size_t)n);
-		on_threads(n - 1, [&](uint64_t lo, uint64_t hi) {
-			for (uint64_t i = lo; i < hi; ++i)
-				t[(size_t)i + 1] = f((double)(i + 1));
-		});
-		for (uint64_t i = 1; i < n; ++i)
-			sum += t[(size_t)i];
-	} else {
-		const int N = 1 << 16;
-		double a = 1.0, b = (double)(n - 1), dx = (b - a) / N;
-		double integ = f(a) + f(b);
-		std::vector<double> t(N);
-		on_threads(N, [&](uint64_t lo, uint64_t hi) {
-			for (uint64_t j = std::max<uint64_t>(lo, 1); j < hi; ++j)
-				t[j] = f(a + (int)j * dx) * ((j & 1) ? 4.0 : 2.0);
-		});
-		for (int j = 1; j < N; ++j)
-			integ += t[j];
-		integ *= dx / 3.0;
-		sum = integ + 0.5 * (f(a) + f(b));
-	}
-	return sum / (double)n;
+	const unsigned most = std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+	if (n <= (1u << 20))
+		return ordered_sum(1, n, 0.0, most, [&](uint64_t i) { return f((double)i); }) / (double)n;
+	const int N = 1 << 16;
+	const double a = 1.0, b = (double)(n - 1), dx = (b - a) / N;
+	const double integ = ordered_sum(1, N, f(a) + f(b), most, [&](uint64_t j) {
+		return f(a + (int)j * dx) * ((j & 1) ? 4.0 : 2.0);
+	}) * (dx / 3.0);
+	return (integ + 0.5 * (f(a) + f(b))) / (double)n;
 }
 
 } // namespace
