@@ -290,6 +290,9 @@ extern "C" int bbt_make_filter(const char *seq, const uint64_t *offsets, uint64_
 		const unsigned long long fresh_n = cnt[1];
 		cnt[1] = cnt[0] - fresh_n;
 		cnt[0] = fresh_n;
+		/* before the file is opened, which empties one that is there */
+		host.resize(m / 8);
+		MK_TRY(cudaMemcpy(host.data(), d_words, m / 8, cudaMemcpyDeviceToHost));
 		BfHeader hd;
 		hd.m = m;
 		hd.h = h;
@@ -306,8 +309,6 @@ extern "C" int bbt_make_filter(const char *seq, const uint64_t *offsets, uint64_
 			rc = fail(nullptr, BBT_ERR_IO, "cannot write " + bf);
 			goto out;
 		}
-		host.resize(m / 8);
-		MK_TRY(cudaMemcpy(host.data(), d_words, m / 8, cudaMemcpyDeviceToHost));
 		bool ok = write_bf_header(f, hd) == 0 && fwrite(host.data(), 1, host.size(), f) == host.size();
 		ok = (fclose(f) == 0) && ok;
 		if (!ok) {
