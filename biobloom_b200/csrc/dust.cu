@@ -45,6 +45,9 @@
  * but leave the window as it is.
  */
 #include "dust.cuh"
+
+#include <algorithm>
+
 #include "dust_core.cuh"
 
 namespace bbt {
@@ -344,24 +347,35 @@ size_t dust_perfect_bytes()
 	return sizeof(DustPerfect);
 }
 
+/* Shared memory of a block of nt threads of pass 0; above kDustPass0Block a block
+ * has fewer threads. */
+static size_t dust_pass0_bytes(unsigned nt, int W)
+{
+	return (size_t)nt * (64 * 4 + (size_t)(W - 2) * 2);
+}
+constexpr size_t kDustPass0Block = 56u << 10;
+
 cudaError_t launch_dust_pass1(const DustArgs &a, int num_sms, cudaStream_t s)
 {
 	const uint64_t total = a.n * a.mates;
 	if (total == 0)
 		return cudaSuccess;
-	/* threads per block: as many as keep four blocks on an SM, from 32 (W = 1024:
-	 * 74 KB) to 128 (W = 64: 49 KB) */
+	/* threads per block: as many as keep four blocks on an SM, from 128 (W = 64:
+	 * 47.5 KB) down to 32, of which three fit from W = 770 on (W = 1024: 72 KB).  The
+	 * limit is the most that any W takes, not this one's: it belongs to the process,
+	 * where another thread's context may have a larger W. */
 	unsigned nt = 128;
-	auto bytes = [&](unsigned t) { return (size_t)t * (64 * 4 + (size_t)(a.W - 2) * 2); };
-	while (nt > 32 && bytes(nt) > (56u << 10))
+	while (nt > 32 && dust_pass0_bytes(nt, a.W) > kDustPass0Block)
 		nt /= 2;
+	const size_t bytes = dust_pass0_bytes(nt, a.W);
 	cudaError_t e = cudaFuncSetAttribute(dust_pass0_kernel,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(nt));
+			cudaFuncAttributeMaxDynamicSharedMemorySize,
+			(int)std::max(kDustPass0Block, dust_pass0_bytes(32, kDustMaxWindow)));
 	if (e != cudaSuccess)
 		return e;
 	const uint64_t need = (total + nt - 1) / nt;
 	const uint64_t cap = (uint64_t)num_sms * 64;
-	dust_pass0_kernel<<<(unsigned)(need < cap ? need : cap), nt, bytes(nt), s>>>(a);
+	dust_pass0_kernel<<<(unsigned)(need < cap ? need : cap), nt, bytes, s>>>(a);
 	if ((e = cudaGetLastError()) != cudaSuccess)
 		return e;
 	/* a full grid: how many reads are listed is known on the device */

@@ -1945,8 +1945,10 @@ template <int H>
 static cudaError_t launch_scan_h(const MibfArgs &a, const ScanLists &l, int num_sms, cudaStream_t s)
 {
 	const size_t smem = scan_smem(a.f.nids);
+	/* the limit of the most IDs, not of these: it belongs to the process, where
+	 * another thread's context may have more */
 	cudaError_t e = cudaFuncSetAttribute(mibf_scan_kernel<H>,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem(kMibfSmemIds));
 	int nb = 0;
 	if (e == cudaSuccess)
 		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mibf_scan_kernel<H>, kScanThreads,
