@@ -184,7 +184,6 @@ extern "C" int bbt_close(bbt_ctx *ctx)
 	cudaFree(ctx->d_dust_scratch);
 	cudaFree(ctx->d_counts);
 	bf_scratch_free(ctx->sc);
-	cudaFree(ctx->d_bthres);
 	cudaFree(ctx->d_lenset);
 	cudaFree(ctx->d_stat);
 	cudaFree(ctx->d_tmp_hits[0]);
@@ -608,9 +607,9 @@ static int bt_grow(bbt_ctx *ctx, uint64_t rows)
 	uint32_t *d = nullptr;
 	CUDA_TRY(ctx, cudaDeviceSynchronize()); /* no kernel may still read the old table */
 	CUDA_TRY(ctx, cudaMalloc(&d, h.size() * 4));
+	std::shared_ptr<uint32_t> table(d, [](uint32_t *p) { cudaFree(p); });
 	CUDA_TRY(ctx, cudaMemcpy(d, h.data(), h.size() * 4, cudaMemcpyHostToDevice));
-	cudaFree(ctx->d_bthres);
-	ctx->d_bthres = d;
+	ctx->bthres = table; /* the old one goes with the last graph that reads it */
 	ctx->h_bthres.swap(h);
 	ctx->bt_have.resize(rows, 0);
 	ctx->bt_rows = rows;
@@ -653,7 +652,7 @@ static int ensure_bthres(bbt_ctx *ctx, const std::vector<uint64_t> &lens)
 			if (L < k)
 				continue;
 			const size_t at = (size_t)f * ctx->bt_rows + (L - k + 1);
-			CUDA_TRY(ctx, cudaMemcpy(ctx->d_bthres + at, &ctx->h_bthres[at], 4,
+			CUDA_TRY(ctx, cudaMemcpy(ctx->bthres.get() + at, &ctx->h_bthres[at], 4,
 					cudaMemcpyHostToDevice));
 		}
 	}
@@ -732,7 +731,7 @@ static ClassifyArgs base_args(const bbt_ctx *ctx)
 	a.scoring = ctx->p.scoring;
 	a.min_len = (unsigned)std::round(ctx->p.score);
 	a.kmax = ctx->kmax;
-	a.bthres = ctx->d_bthres;
+	a.bthres = ctx->bthres.get();
 	a.bthres_rows = ctx->bt_rows;
 	a.work = ctx->sc.work;
 	a.lane_long = ctx->lc.steps == BBT_STEPS_DECISION &&
@@ -2276,6 +2275,7 @@ struct bbt_graph {
 	cudaGraph_t graph = nullptr;
 	cudaGraphExec_t exec = nullptr;
 	cudaStream_t capture = nullptr;
+	std::shared_ptr<uint32_t> bthres; /* the threshold table that the launches read */
 	BfScratch sc; /* what the captured launches use: a later call on the context may
 	                 replace the buffers of the context's own */
 	uint64_t reads = 0, launches = 0;
@@ -2337,6 +2337,7 @@ extern "C" int bbt_graph_create(bbt_ctx *ctx, const bbt_batch *b, const bbt_resu
 		bbt_graph_destroy(g);
 		return rc;
 	}
+	g->bthres = ctx->bthres;
 	std::swap(ctx->sc, g->sc);
 	ctx->capturing = true;
 	cudaError_t e = cudaStreamCreateWithFlags(&g->capture, cudaStreamNonBlocking);

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -124,7 +125,7 @@ struct bbt_ctx {
 	std::mutex bt_mu;
 	std::vector<uint32_t> h_bthres;  /* nf x bt_rows */
 	std::vector<uint8_t> bt_have;    /* by read length */
-	uint32_t *d_bthres = nullptr;
+	std::shared_ptr<uint32_t> bthres; /* on the device; a captured graph keeps the one it reads */
 	uint64_t bt_rows = 0;
 	unsigned int *d_lenset = nullptr;
 	bool capturing = false;          /* a CUDA graph is being captured */

@@ -385,7 +385,9 @@ int bbt_set_steps(bbt_ctx *ctx, int steps);
  * graph is bound to the batch's and results' device pointers: refill those
  * buffers between launches.  It holds what else its launches use: other calls
  * on the context may come between them, of any size (BESTHIT graphs hold up to
- * 1 GB for their scores).  Summary counters are updated at each launch.
+ * 1 GB for their scores).  With BINOMIAL scoring the reads that it is replayed
+ * on must have lengths of the captured batch's (their thresholds are computed
+ * before the capture).  Summary counters are updated at each launch.
  * Plain and persistent paths only (the filter-major path reads block sums on
  * the host).  Create it after a warm-up call with the same sizes.
  */

@@ -54,3 +54,33 @@ def test_replays_after_larger_calls(tmp_path, mode, paired, n, schedule, first):
             for h, m in zip(got, more):
                 assert np.array_equal(h.cpu().numpy().view(np.uint64), want(m))
         g.close()
+
+
+def test_binomial_thresholds_outlive_a_larger_table(tmp_path):
+    """A call with longer reads replaces the context's threshold table; the graph reads on in
+    the one it was captured with."""
+    import torch
+    rng = np.random.default_rng(17)
+    genomes, filters, paths = _filters(tmp_path, rng, [25, 21], 3)
+    reads = [genomes[0][i:i + 150].tobytes() for i in range(400)] + \
+        [rng.choice(genomes[0], 150).tobytes() for _ in range(400)]
+    longer = [genomes[1][:9000].tobytes(), rng.choice(genomes[1], 5000).tobytes()]
+    want = [ol.classify(*ol.pack_reads(r), filters, 10.0 ** -10.0, 3, scoring=ol.BINOMIAL)[0]
+            for r in (reads, longer)]
+    dev, dev_longer = _device(reads), _device(longer)
+    hits = torch.empty((len(reads), 1), dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    with _open(paths, ol.BINOMIAL, 100, 3, path=2) as bbc:
+        g = bbc.graph(*dev, hits)
+        for _ in range(2):
+            got = bbc.classify_device(*dev_longer)[0]
+            torch.cuda.synchronize()
+            assert np.array_equal(got.cpu().numpy().view(np.uint64), want[1])
+            taken = torch.full((1 << 22,), -1, dtype=torch.int32, device="cuda")  # over freed memory
+            hits.fill_(-1)
+            torch.cuda.synchronize()
+            g.launch()
+            torch.cuda.synchronize()
+            assert np.array_equal(hits.cpu().numpy().view(np.uint64), want[0])
+            del taken
+        g.close()
