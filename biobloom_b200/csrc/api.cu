@@ -734,8 +734,9 @@ static ClassifyArgs base_args(const bbt_ctx *ctx)
 	a.bthres = ctx->bthres.get();
 	a.bthres_rows = ctx->bt_rows;
 	a.work = ctx->sc.work;
-	a.lane_long = ctx->lc.steps == BBT_STEPS_DECISION &&
-			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, 0);
+	if (ctx->lc.steps == BBT_STEPS_DECISION &&
+			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, 0))
+		a.long_bases = kWindowBases;
 	if (ctx->lc.count) {
 		a.probes = ctx->d_stat;
 		a.frames = ctx->d_stat + 1;

@@ -46,8 +46,9 @@ struct ClassifyArgs {
 	int tight_steps;           /* SIMPLE scoring: size probe steps by the frames that could
 	                              still accept the read (seqeval_chunk.cuh,
 	                              simple_step_frames) instead of 32 frames per step */
-	int lane_long;             /* persistent path: long reads in windows of up to 256 frames
-	                              (lane_long_item; filters and options as lane_supports) */
+	uint32_t long_bases;       /* persistent path: reads above this many bases in windows of up
+	                              to 256 frames (lane_long_item; filters and options as
+	                              lane_supports); 0: none */
 	unsigned long long *probes;/* optional: filter words read */
 	unsigned long long *frames;/* optional: frames hashed */
 	unsigned long long *alg_probes; /* optional: words the sequential algorithm reads */
