@@ -184,6 +184,7 @@ extern "C" int bbt_close(bbt_ctx *ctx)
 	cudaFree(ctx->d_dust_scratch);
 	cudaFree(ctx->d_counts);
 	bf_scratch_free(ctx->sc);
+	cudaFreeHost(ctx->h_lane_stats);
 	cudaFree(ctx->d_lenset);
 	cudaFree(ctx->d_stat);
 	cudaFree(ctx->d_tmp_hits[0]);
@@ -525,6 +526,7 @@ extern "C" int bbt_open(const char *const *bf_paths, int n_filters, const bbt_pa
 	OPEN_TRY(cudaMalloc(&ctx->d_counts, sizeof(unsigned long long) * (2 * (ctx->nf + 2) + 2)));
 	OPEN_TRY(cudaMemset(ctx->d_counts, 0, sizeof(unsigned long long) * (2 * (ctx->nf + 2) + 2)));
 	OPEN_TRY(scratch_counters(ctx, ctx->sc));
+	OPEN_TRY(cudaMallocHost(&ctx->h_lane_stats, kLaneStats * sizeof(unsigned long long)));
 	OPEN_TRY(cudaMalloc(&ctx->d_stat, 3 * sizeof(unsigned long long)));
 	OPEN_TRY(cudaMemset(ctx->d_stat, 0, 3 * sizeof(unsigned long long)));
 	ctx->cap_reads = ctx->p.max_batch_reads ? ctx->p.max_batch_reads : (1ull << 20);
@@ -1225,16 +1227,23 @@ static int dust_check(bbt_ctx *ctx)
 	return BBT_OK;
 }
 
-/* Whether these launches take the lane kernel: the persistent path with its
- * default steps and the filter-major path, with filters and options that it
- * supports, for enough reads. */
-static bool lane_wanted(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t total)
+/* Who takes a batch: the warp kernels, the lane kernel, or the one that the lengths
+ * of its reads ask for (ClassifyArgs::lane_stats). */
+enum LaneUse { kLaneNo, kLaneYes, kLaneAsk };
+
+/* The persistent path with its default steps and the filter-major path, with filters
+ * and options that the lane kernel supports, for enough reads. */
+static LaneUse lane_use(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t total, LaneRule &rule)
 {
-	const bool path = lc.path == BBT_PATH_FILTER_MAJOR ||
-			(lc.path == BBT_PATH_PERSISTENT && lc.steps == BBT_STEPS_DECISION);
-	const bool scores = ctx->mode == BBT_MODE_BESTHIT || ctx->mode == BBT_MODE_SCORES;
-	return path && lane_pays(ctx->hf.data(), ctx->nf, total, scores) &&
-			lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total);
+	if (lc.path != BBT_PATH_FILTER_MAJOR &&
+			!(lc.path == BBT_PATH_PERSISTENT && lc.steps == BBT_STEPS_DECISION))
+		return kLaneNo;
+	rule = lane_rule(ctx->hf.data(), ctx->nf, ctx->mode == BBT_MODE_BESTHIT ||
+			ctx->mode == BBT_MODE_SCORES, total);
+	if (total < rule.least ||
+			!lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total))
+		return kLaneNo;
+	return total < rule.sure ? kLaneAsk : kLaneYes;
 }
 
 /* BESTHIT by the lane kernel goes through stored scores: outside the
@@ -1246,11 +1255,17 @@ static bool lane_stores_scores(const bbt_ctx *ctx, uint64_t n, uint32_t mates)
 			n * ctx->nf * mates <= (128ull << 20);
 }
 
-/* The lane kernel over a batch: hits (classify) and / or scores (sa). */
+static LaneScratch lane_scratch(const BfScratch &sc)
+{
+	return {sc.lane_list, sc.order_cnt + kOrderCounters};
+}
+
+/* The lane kernel over a batch whose lengths are listed: hits (classify) and / or
+ * scores (sa). */
 static int run_lane(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreArgs *sa,
 		bool classify)
 {
-	const LaneScratch ls = {ctx->sc.lane_list, ctx->sc.order_cnt};
+	const LaneScratch ls = lane_scratch(ctx->sc);
 	const bool count = ctx->lc.count != 0;
 	const bool both = classify && sa && !count; /* one walk for hits and scores */
 	if (classify) {
@@ -1260,12 +1275,53 @@ static int run_lane(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreAr
 	}
 	if (classify && !both) {
 		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, true, ls, ctx->num_sms, count, s));
-		ctx->last.kernels += 1 + ctx->nf;
+		ctx->last.kernels += ctx->nf;
 	}
 	if (sa) {
 		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), sa, both, ls, ctx->num_sms, false, s));
-		ctx->last.kernels += 1 + ctx->nf;
+		ctx->last.kernels += ctx->nf;
 	}
+	return BBT_OK;
+}
+
+/* The read-major kernels over a batch: hits (classify), in the read order if one is
+ * set, and / or scores (sa). */
+static int run_warps(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreArgs *sa,
+		bool classify)
+{
+	if (classify) {
+		LaunchConfig lc = ctx->lc;
+		if (lc.path == BBT_PATH_FILTER_MAJOR)
+			lc.path = BBT_PATH_PERSISTENT; /* filters of different k */
+		if (lc.path != BBT_PATH_PLAIN)
+			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.work, 0, sizeof(unsigned long long), s));
+		if (lc.path != BBT_PATH_PLAIN && ctx->long_bases) {
+			int rc = grow(ctx, &ctx->sc.order, ctx->sc.order_cap, a.n * a.mates);
+			if (rc)
+				return rc;
+			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.order_cnt, 0,
+					kOrderCounters * sizeof(unsigned long long), s));
+			CUDA_TRY(ctx, launch_long_first(a, ctx->long_bases, ctx->sc.order, ctx->sc.order_cnt,
+					ctx->num_sms, s));
+			a.order = ctx->sc.order;
+			ctx->last.kernels += 1;
+		}
+		CUDA_TRY(ctx, launch_classify(a, lc, s));
+		ctx->last.kernels += 1;
+	}
+	if (sa) {
+		CUDA_TRY(ctx, launch_scores(a, *sa, ctx->lc, s));
+		ctx->last.kernels += 1;
+	}
+	return BBT_OK;
+}
+
+/* Zeroed hit words, which the filter-major passes OR an accepted item's bit into. */
+static int zero_hits(bbt_ctx *ctx, const ClassifyArgs &a, cudaStream_t s)
+{
+	const size_t hb = a.n * ctx->words * sizeof(uint64_t);
+	for (uint32_t m = 0; m < a.mates; ++m)
+		CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
 	return BBT_OK;
 }
 
@@ -1274,7 +1330,7 @@ static int run_lane(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreAr
 static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStream_t s,
 		double *const *scores = nullptr, const uint64_t *mate_bases = nullptr)
 {
-	ctx->last.kernels = 2; /* classification (counted below for two-pass) + summary */
+	ctx->last.kernels = 1; /* the summary; what follows counts itself */
 	if (ctx->dust) {
 		if (!mate_bases)
 			return fail(ctx, BBT_ERR_UNSUPPORTED, "DUST masking needs the batch's base counts");
@@ -1287,105 +1343,79 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	sa.scores[1] = scores && a.mates == 2 ? scores[1] : nullptr;
 	sa.fpr = ctx->d_fpr;
 	sa.besthit = 0;
-	bool want_scores = sa.scores[0] || sa.scores[1];
+	const bool want_scores = sa.scores[0] || sa.scores[1];
+	const bool best = ctx->mode == BBT_MODE_BESTHIT;
+	const bool best_only = best && !want_scores;
 	const bool two_pass = ctx->lc.path == BBT_PATH_FILTER_MAJOR && ctx->same_k;
-	const bool best_only = ctx->mode == BBT_MODE_BESTHIT && !want_scores;
-	bool lane = lane_wanted(ctx, ctx->lc, a.n * a.mates);
+	LaneRule rule;
+	LaneUse lane = lane_use(ctx, ctx->lc, a.n * a.mates, rule);
 	if (lane && best_only && !lane_stores_scores(ctx, a.n, a.mates))
-		lane = false;
+		lane = kLaneNo;
 	/* scores of one mate only: the kernels that test each array */
 	if (lane && want_scores && (!sa.scores[0] || (a.mates == 2 && !sa.scores[1])))
-		lane = false;
+		lane = kLaneNo;
 	/* no allocation while a graph is captured: with the scratch that it has */
 	if (lane && ctx->capturing && (a.n * a.mates > ctx->sc.lane_list_cap ||
 			(best_only && a.n * ctx->nf > ctx->sc.scores_cap)))
-		lane = false;
+		lane = kLaneNo;
 	if (lane) {
 		int rc = grow(ctx, &ctx->sc.lane_list, ctx->sc.lane_list_cap, a.n * a.mates);
 		if (rc)
 			return rc;
 	}
 	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_k0, s));
-	if ((lane || two_pass) && (ctx->mode == BBT_MODE_BESTHIT || want_scores)) {
-		/* filter-major score pass (and filter pass for the hits unless
-		 * BESTHIT, whose hits come from the scores) */
-		ScoreArgs ps = sa;
-		if (best_only) {
-			const uint64_t need = a.n * ctx->nf;
-			if (need > ctx->sc.scores_cap) {
-				cudaFree(ctx->sc.scores[0]);
-				cudaFree(ctx->sc.scores[1]);
-				ctx->sc.scores[0] = ctx->sc.scores[1] = nullptr;
-				ctx->sc.scores_cap = 0;
-				CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[0], need * sizeof(double)));
-				CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[1], need * sizeof(double)));
-				ctx->sc.scores_cap = need;
-			}
-			ps.scores[0] = ctx->sc.scores[0];
-			ps.scores[1] = a.mates == 2 ? ctx->sc.scores[1] : nullptr;
+	if (lane) {
+		const LaneScratch ls = lane_scratch(ctx->sc);
+		CUDA_TRY(ctx, launch_lane_list(a, ls, ctx->num_sms, s));
+		ctx->last.kernels += 1;
+		if (lane == kLaneAsk && two_pass) {
+			/* these passes are planned on the host, with a short wait: so is the choice */
+			CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_lane_stats, ls.ctr, kLaneStats *
+					sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
+			CUDA_TRY(ctx, cudaStreamSynchronize(s));
+			lane = lane_takes(rule, ctx->h_lane_stats, a.n * a.mates) ? kLaneYes : kLaneNo;
+		} else if (lane == kLaneAsk) {
+			a.lane_stats = ls.ctr;
+			a.lane_rule = rule;
 		}
-		const bool classify = ctx->mode != BBT_MODE_BESTHIT;
-		if (classify && !lane) {
-			const size_t hb = a.n * ctx->words * sizeof(uint64_t);
-			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[0], 0, hb, s));
-			if (a.mates == 2)
-				CUDA_TRY(ctx, cudaMemsetAsync(a.hits[1], 0, hb, s));
-		}
-		ctx->last.kernels -= 1; /* the passes count themselves */
-		int rc = lane ? run_lane(ctx, a, s, &ps, classify) : run_two_pass(ctx, a, s, &ps, classify);
-		if (rc)
-			return rc;
-		if (!classify) {
-			CUDA_TRY(ctx, launch_best_hits(a, ps.scores, ctx->num_sms, s));
-			ctx->last.kernels += 1;
-		}
-		want_scores = false; /* done */
-	} else if (ctx->mode == BBT_MODE_BESTHIT) {
-		/* the hit words are the filters of the largest score */
-		sa.besthit = 1;
-		CUDA_TRY(ctx, launch_scores(a, sa, ctx->lc, s));
-	} else if (ctx->lc.path == BBT_PATH_BUCKETED && !want_scores) {
-		ctx->last.kernels -= 1; /* the passes count themselves */
-		int rc = run_bucketed(ctx, a, s);
-		if (rc)
-			return rc;
-	} else if (lane) {
-		ctx->last.kernels -= 1;
-		int rc = run_lane(ctx, a, s, nullptr, true);
-		if (rc)
-			return rc;
-	} else if (two_pass) {
-		/* accepted (filter, read) items OR their bit into zeroed words */
-		const size_t hb = a.n * ctx->words * sizeof(uint64_t);
-		CUDA_TRY(ctx, cudaMemsetAsync(a.hits[0], 0, hb, s));
-		if (a.mates == 2)
-			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[1], 0, hb, s));
-		ctx->last.kernels -= 1; /* the passes count themselves */
-		int rc = run_two_pass(ctx, a, s);
-		if (rc)
-			return rc;
-	} else {
-		LaunchConfig lc = ctx->lc;
-		if (lc.path == BBT_PATH_FILTER_MAJOR)
-			lc.path = BBT_PATH_PERSISTENT; /* filters of different k */
-		if (lc.path != BBT_PATH_PLAIN)
-			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.work, 0, sizeof(unsigned long long), s));
-		if (lc.path != BBT_PATH_PLAIN && ctx->long_bases) {
-			int rc = grow(ctx, &ctx->sc.order, ctx->sc.order_cap, a.n * a.mates);
-			if (rc)
-				return rc;
-			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.order_cnt, 0, 2 * sizeof(unsigned long long), s));
-			CUDA_TRY(ctx, launch_long_first(a, ctx->long_bases, ctx->sc.order, ctx->sc.order_cnt,
-					ctx->num_sms, s));
-			a.order = ctx->sc.order;
-			ctx->last.kernels += 1;
-		}
-		CUDA_TRY(ctx, launch_classify(a, lc, s));
 	}
-	if (want_scores && ctx->mode != BBT_MODE_BESTHIT) {
-		CUDA_TRY(ctx, launch_scores(a, sa, ctx->lc, s));
+	/* the scores that BESTHIT's hits come from, where nobody asked for them */
+	ScoreArgs ps = sa;
+	if (best_only && (lane || two_pass)) {
+		const uint64_t need = a.n * ctx->nf;
+		if (need > ctx->sc.scores_cap) {
+			cudaFree(ctx->sc.scores[0]);
+			cudaFree(ctx->sc.scores[1]);
+			ctx->sc.scores[0] = ctx->sc.scores[1] = nullptr;
+			ctx->sc.scores_cap = 0;
+			CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[0], need * sizeof(double)));
+			CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[1], need * sizeof(double)));
+			ctx->sc.scores_cap = need;
+		}
+		ps.scores[0] = ctx->sc.scores[0];
+		ps.scores[1] = a.mates == 2 ? ctx->sc.scores[1] : nullptr;
+	}
+	const bool stored = best || want_scores; /* scores go to memory (lane, two-pass) */
+	int rc = BBT_OK;
+	if (lane) {
+		rc = run_lane(ctx, a, s, stored ? &ps : nullptr, !best);
+	} else if (two_pass) {
+		rc = best ? BBT_OK : zero_hits(ctx, a, s);
+		if (!rc)
+			rc = run_two_pass(ctx, a, s, stored ? &ps : nullptr, !best);
+	}
+	if (!rc && best && (lane || two_pass)) {
+		CUDA_TRY(ctx, launch_best_hits(a, ps.scores, ctx->num_sms, s));
 		ctx->last.kernels += 1;
 	}
+	if (!rc && lane != kLaneYes && !two_pass) {
+		/* the hit words of BESTHIT are the filters of the largest score */
+		sa.besthit = best;
+		const bool bucketed = ctx->lc.path == BBT_PATH_BUCKETED && !stored;
+		rc = bucketed ? run_bucketed(ctx, a, s) : run_warps(ctx, a, s, stored ? &sa : nullptr, !best);
+	}
+	if (rc)
+		return rc;
 	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_k1, s));
 	CUDA_TRY(ctx, launch_summarize(a.hits[0], a.mates == 2 ? a.hits[1] : nullptr, a.n, ctx->nf,
 			ctx->words, ctx->p.inclusive, ctx->mode == BBT_MODE_ORDERED, d_cat, ctx->d_counts,
@@ -2293,7 +2323,8 @@ static int graph_scratch(bbt_ctx *ctx, BfScratch &sc, uint64_t reads, uint32_t m
 		if (rc)
 			return rc;
 	}
-	if (lane_wanted(ctx, ctx->lc, reads * mates) &&
+	LaneRule rule;
+	if (lane_use(ctx, ctx->lc, reads * mates, rule) &&
 			grow_if_room(&sc.lane_list, sc.lane_list_cap, reads * mates) &&
 			ctx->mode == BBT_MODE_BESTHIT && lane_stores_scores(ctx, reads, mates)) {
 		uint64_t cap[2] = {0, 0};
@@ -2421,6 +2452,8 @@ int bbt::bf_scratch_init(bbt_ctx *ctx, BfScratch &sc, uint64_t max_reads)
 	CUDA_TRY(ctx, scratch_counters(ctx, sc));
 	CUDA_TRY(ctx, cudaMalloc(&sc.order, std::max<uint64_t>(max_reads, 1) * 2 * sizeof(uint64_t)));
 	sc.order_cap = std::max<uint64_t>(max_reads, 1) * 2;
+	CUDA_TRY(ctx, cudaMalloc(&sc.lane_list, sc.order_cap * sizeof(uint32_t)));
+	sc.lane_list_cap = sc.order_cap;
 	return BBT_OK;
 }
 
@@ -2459,31 +2492,41 @@ int bbt::bf_classify_slot(bbt_ctx *ctx, const uint8_t *seq, const uint64_t *off,
 	lc.count = 0;
 	if (lc.path == BBT_PATH_FILTER_MAJOR)
 		lc.path = BBT_PATH_PERSISTENT;
-	const bool lane = ctx->mode != BBT_MODE_BESTHIT && n * a.mates <= sc.order_cap &&
-			lane_wanted(ctx, lc, n * a.mates);
-	if (lane) {
-		const size_t hb = n * ctx->words * sizeof(uint64_t);
-		for (uint32_t m = 0; ctx->nf > 1 && m < a.mates; ++m)
-			CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
-		const LaneScratch ls = {reinterpret_cast<uint32_t *>(sc.order), sc.order_cnt};
-		CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, true, ls, ctx->num_sms, false, s));
-	} else if (ctx->mode == BBT_MODE_BESTHIT) {
+	if (ctx->mode == BBT_MODE_BESTHIT) {
 		ScoreArgs sa;
 		sa.scores[0] = sa.scores[1] = nullptr;
 		sa.fpr = ctx->d_fpr;
 		sa.besthit = 1;
 		CUDA_TRY(ctx, launch_scores(a, sa, lc, s));
-	} else if (lc.path != BBT_PATH_PLAIN) {
-		CUDA_TRY(ctx, cudaMemsetAsync(sc.work, 0, sizeof(unsigned long long), s));
-		if (ctx->long_bases && n * a.mates <= sc.order_cap) {
-			CUDA_TRY(ctx, cudaMemsetAsync(sc.order_cnt, 0, 2 * sizeof(unsigned long long), s));
-			CUDA_TRY(ctx, launch_long_first(a, ctx->long_bases, sc.order, sc.order_cnt,
-					ctx->num_sms, s));
-			a.order = sc.order;
+	} else {
+		LaneRule rule;
+		const LaneUse lane = n * a.mates <= sc.lane_list_cap ? lane_use(ctx, lc, n * a.mates, rule)
+		                                                     : kLaneNo;
+		if (lane) {
+			const LaneScratch ls = lane_scratch(sc);
+			CUDA_TRY(ctx, launch_lane_list(a, ls, ctx->num_sms, s));
+			if (lane == kLaneAsk) {
+				a.lane_stats = ls.ctr;
+				a.lane_rule = rule;
+			}
+			const size_t hb = n * ctx->words * sizeof(uint64_t);
+			for (uint32_t m = 0; ctx->nf > 1 && m < a.mates; ++m)
+				CUDA_TRY(ctx, cudaMemsetAsync(a.hits[m], 0, hb, s));
+			CUDA_TRY(ctx, launch_lane(a, ctx->hf.data(), nullptr, true, ls, ctx->num_sms, false, s));
 		}
+		if (lane != kLaneYes && lc.path != BBT_PATH_PLAIN) {
+			CUDA_TRY(ctx, cudaMemsetAsync(sc.work, 0, sizeof(unsigned long long), s));
+			if (ctx->long_bases && n * a.mates <= sc.order_cap) {
+				CUDA_TRY(ctx, cudaMemsetAsync(sc.order_cnt, 0,
+						kOrderCounters * sizeof(unsigned long long), s));
+				CUDA_TRY(ctx, launch_long_first(a, ctx->long_bases, sc.order, sc.order_cnt,
+						ctx->num_sms, s));
+				a.order = sc.order;
+			}
+		}
+		if (lane != kLaneYes)
+			CUDA_TRY(ctx, launch_classify(a, lc, s));
 	}
-	if (ctx->mode != BBT_MODE_BESTHIT && !lane)
-		CUDA_TRY(ctx, launch_classify(a, lc, s));
 	CUDA_TRY(ctx, launch_summarize(a.hits[0], paired ? a.hits[1] : nullptr, n, ctx->nf,
 			ctx->words, ctx->p.inclusive, ctx->mode == BBT_MODE_ORDERED, category,
 			ctx->d_counts, ctx->num_sms, s));

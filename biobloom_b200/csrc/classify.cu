@@ -247,6 +247,8 @@ __global__ void __launch_bounds__(256, BBT_CLASSIFY_MIN_BLOCKS) classify_kernel(
 		const __grid_constant__ ClassifyArgs a)
 {
 	extern __shared__ __align__(16) unsigned char smem[];
+	if (a.lane_stats && lane_has(a))
+		return;
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	const Window<SEG> win = window_at<SEG>(smem + warp * window_stride<SEG>(a.kmax));

@@ -15,6 +15,17 @@
 
 namespace bbt {
 
+/* Which batches the lane kernel (lane.cu) takes: none of fewer reads than `least`,
+ * all from `sure` reads on, and between these what lane_takes (lane.cuh) makes of
+ * their lengths and the limits below. */
+struct LaneRule {
+	uint64_t least, sure;
+	uint32_t mids, longs; /* at most one read in so many has 385 to 1024 bases, or more than
+	                         that (0: any number) */
+	uint32_t mean;        /* mean length of the reads up to 384 bases, at most */
+	bool even;            /* and at least 4/5 of the longest one's */
+};
+
 /* Everything one classify launch needs.  Reads r in [0, n * mates): r < n is
  * read r of mate array 0, otherwise read r - n of mate array 1. */
 struct ClassifyArgs {
@@ -49,6 +60,11 @@ struct ClassifyArgs {
 	uint32_t long_bases;       /* persistent path: reads above this many bases in windows of up
 	                              to 256 frames (lane_long_item; filters and options as
 	                              lane_supports); 0: none */
+	const unsigned long long *lane_stats; /* when given, the batch's lengths as lane_list_kernel
+	                              counted them decide on the device: the lane kernel and the
+	                              warp kernels are both launched, and the ones that
+	                              lane_rule does not name end at once */
+	LaneRule lane_rule;
 	unsigned long long *probes;/* optional: filter words read */
 	unsigned long long *frames;/* optional: frames hashed */
 	unsigned long long *alg_probes; /* optional: words the sequential algorithm reads */

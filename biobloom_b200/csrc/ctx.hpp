@@ -49,10 +49,11 @@ struct Slot {
 
 void set_global_error(const std::string &msg);
 
-/* Counters of the read order (2) or of the lane kernel. */
+/* Counters of the read order, then those of the lane kernel: one batch may use both. */
+constexpr size_t kOrderCounters = 2;
 inline size_t order_counters(uint32_t nf)
 {
-	return std::max<size_t>(2, lane_counters(nf));
+	return kOrderCounters + lane_counters(nf);
 }
 
 /* Device scratch of classification calls that run one after another.  The
@@ -87,6 +88,7 @@ struct bbt_ctx {
 	uint32_t nf = 0, words = 0, kmax = 0;
 	unsigned long long *d_counts = nullptr; /* 2*(nf+2)+2 summary counters */
 	bbt::BfScratch sc;
+	unsigned long long *h_lane_stats = nullptr; /* pinned: a batch's lengths (lane.cuh) */
 	unsigned long long *d_stat = nullptr;   /* probes, frames */
 	uint64_t reads_seen = 0;
 	bbt::Slot slot[2];

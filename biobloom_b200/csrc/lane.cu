@@ -18,9 +18,13 @@
  * one filter at a time and a filter that fits L2 stays there; warps take chunks
  * of 32 reads from a counter.  A warp keeps its next items (base position,
  * length, thresholds: computed 32 at a time) in shared memory and hands them to
- * lanes as these finish.  Reads above LaneArgs::max_bases would leave a lane working
- * long after its warp and are evaluated by whole warps, before the others: a
- * small kernel lists them.
+ * lanes as these finish.  Reads above 1024 bases, and most above 384 (lane_mids),
+ * would leave a lane working long after its warp and are evaluated by whole warps,
+ * before the others: a small kernel lists them.  The grid is full whatever the batch,
+ * for the list (28,000 listed reads of 600 bases with one warp a chunk, 880 warps:
+ * 680 us against 351), and chunks are handed to a part of each block (LaneShare): left
+ * to the warps that come first they end up on some of the SMs (20,000 reads of 150
+ * bases over a 3.4 MB filter 140 us against 95).
  */
 #include "lane.cuh"
 
@@ -35,7 +39,7 @@ namespace {
 
 constexpr int kLaneWarps = 8;     /* warps per block */
 /* Blocks per SM the registers leave room for: 3 give a thread 80, which hold
- * eight frames' hashes and words in flight without spills (4 blocks spill, and
+ * eight frames' hashes and words in flight (with 4 blocks the steps spill, and
  * the spilled words cost more L2 and L1 than the warps bring: 11.8 against 10.1
  * ms on the ten 68 MB filters). */
 constexpr int kLaneMinBlocks = 3;
@@ -51,12 +55,11 @@ struct LaneArgs {
 	ClassifyArgs a;
 	ScoreArgs sa;
 	const uint32_t *list;
-	const unsigned long long *nlong;
-	unsigned long long *ctr;    /* next chunk, next long read */
+	const unsigned long long *stats;
+	unsigned long long *ctr;    /* next chunk, next listed read */
 	uint64_t chunks;
 	uint32_t f;                 /* the filter's index */
 	LaneFilter F;
-	uint32_t max_bases;         /* of a lane's read */
 };
 
 /* What a lane needs of its read once per eight bases or less, and the bases
@@ -70,41 +73,108 @@ struct LaneWarp {
 	uint32_t my_read[32], my_len[32];
 	int32_t my_thres[32], my_anti_thres[32];
 	uint32_t nib[4][32];        /* nibbles of the last 32 bases, 8 to a word */
+	uint32_t first;             /* the next chunk is the warp's own */
 	double hthres[MODE == SCORE_HARMONIC ? 32 : 1], my_hthres[MODE == SCORE_HARMONIC ? 32 : 1];
 };
 
-/* Indexes of the reads above max_bases. */
-__global__ void lane_long_kernel(ClassifyArgs a, uint32_t max_bases, uint32_t *list,
-		unsigned long long *nlong)
+/* What a block's warps make of the batch's lengths.  Of a batch with fewer chunks than
+ * warps, the first warps of each block take them, so that the SMs share them evenly:
+ * without listed reads each its own first one, the others from the counter.  The
+ * warps that have no chunks join in on the list only where it is long (more than
+ * four reads a chunk): the longest reads, which the launch waits for, go faster
+ * without (50,000 ragged reads over 2.1 GB, 2,500 of them listed: 404 us against
+ * 436). */
+struct LaneShare {
+	uint32_t nlong, listed;     /* listed reads above kLaneMaxBases, and all */
+	uint32_t max_bases;         /* of a lane's read */
+	uint32_t warps;             /* of a block that take chunks */
+	uint32_t own;               /* chunks that the counter does not give out */
+	uint32_t help;              /* warps without chunks take listed reads */
+	uint32_t go;                /* the batch is this kernel's */
+};
+
+/* The reads above kLaneShortBases (LaneScratch::list) and the counts of the
+ * batch's lengths. */
+__global__ void __launch_bounds__(256) lane_list_kernel(ClassifyArgs a, uint32_t *list,
+		unsigned long long *stats)
 {
+	__shared__ uint64_t sums[8];
+	__shared__ uint32_t tops[8];
 	const uint64_t total = a.n * a.mates;
 	const int lane = threadIdx.x & 31;
+	const unsigned below = (1u << lane) - 1u;
 	const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+	uint32_t bases = 0, longest = 0; /* this thread's reads: at most 2^32 / stride of them */
 	for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < total; base += stride) {
 		const uint64_t r = base + threadIdx.x;
-		bool is_long = false;
+		uint64_t len = 0;
 		if (r < total) {
 			const uint32_t mate = r >= a.n ? 1u : 0u;
 			const uint64_t i = r - (mate ? a.n : 0);
-			is_long = a.off[mate][i + 1] - a.off[mate][i] > max_bases;
+			len = a.off[mate][i + 1] - a.off[mate][i];
 		}
-		const unsigned m = __ballot_sync(kFull, is_long);
-		if (m) {
-			unsigned long long b = 0;
-			if (lane == 0)
-				b = atomicAdd(nlong, (unsigned long long)__popc(m));
-			b = __shfl_sync(kFull, b, 0);
-			if (is_long)
-				list[b + __popc(m & ((1u << lane) - 1u))] = (uint32_t)r;
+		if (len <= kLaneShortBases) {
+			bases += (uint32_t)len;
+			longest = max(longest, (uint32_t)len);
+		}
+		const unsigned lm = __ballot_sync(kFull, len > kLaneMaxBases);
+		const unsigned mm = __ballot_sync(kFull, len > kLaneShortBases) & ~lm;
+		if (!(lm | mm))
+			continue;
+		unsigned long long lb = 0, mb = 0;
+		if (lane == 0) {
+			if (lm)
+				lb = atomicAdd(stats + kLaneLong, (unsigned long long)__popc(lm));
+			if (mm)
+				mb = atomicAdd(stats + kLaneMid, (unsigned long long)__popc(mm));
+		}
+		lb = __shfl_sync(kFull, lb, 0);
+		mb = __shfl_sync(kFull, mb, 0);
+		if ((lm >> lane) & 1u)
+			list[lb + __popc(lm & below)] = (uint32_t)r;
+		else if ((mm >> lane) & 1u)
+			list[total - 1 - (mb + __popc(mm & below))] = (uint32_t)r;
+	}
+	const uint64_t sum = __reduce_add_sync(kFull, bases & 0xFFFFu) +
+			((uint64_t)__reduce_add_sync(kFull, bases >> 16) << 16);
+	longest = __reduce_max_sync(kFull, longest);
+	if (lane == 0) {
+		sums[threadIdx.x >> 5] = sum;
+		tops[threadIdx.x >> 5] = longest;
+	}
+	__syncthreads();
+	if (threadIdx.x == 0) {
+		uint64_t all = 0;
+		for (int i = 0; i < 8; ++i) {
+			all += sums[i];
+			longest = max(longest, tops[i]);
+		}
+		if (all) {
+			atomicAdd(stats + kLaneBases, (unsigned long long)all);
+			atomicMax(stats + kLaneLongest, (unsigned long long)longest);
 		}
 	}
 }
 
+/* Whether lanes take the reads of kLaneShortBases to kLaneMaxBases too, rather than
+ * warps from the list: a lane costs a third of the instructions, but the launch then
+ * lasts as long as a lane with the longest of them.  Over a filter in L2, 500,000
+ * ragged reads with 7,000 of these take 902 us by warps and 1087 by lanes, 28,000
+ * reads of 600 bases 351 and 260, 250,000 of them 2481 and 808; over one in HBM
+ * 250,000 ragged reads 1296 and 1519, 160,000 reads of 600 bases 1967 and 1878 (scores,
+ * which walk every frame: 4463 and 4596, 250,000 of 1,000 bases 11669 and 12848). */
+template <bool SCORE>
+__device__ __forceinline__ bool lane_mids(bool in_l2, unsigned long long mids, uint64_t reads)
+{
+	return in_l2 ? mids >= 25000u : !SCORE && mids * 8u > reads;
+}
+
 /* Items of chunk c, reads [32c, 32c + 32), into the warp's queue: those long
- * enough for a frame and not on the long list; the result of a read without
+ * enough for a frame and of at most max_bases; the result of a read without
  * frames is written here.  Returns their number. */
 template <int MODE, int WHAT, bool PACKED>
-__device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, uint64_t c, int lane)
+__device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, uint64_t c,
+		uint32_t max_bases, int lane)
 {
 	constexpr bool SCORE = WHAT != kLaneHits, HITS = WHAT != kLaneScores;
 	const ClassifyArgs &a = g.a;
@@ -129,7 +199,7 @@ __device__ __forceinline__ int lane_queue(const LaneArgs &g, LaneWarp<MODE> &w, 
 		if (HITS && a.nf == 1)
 			a.hits[mate][i] = 0;
 	}
-	const bool mine = in && l >= g.F.k && l <= g.max_bases;
+	const bool mine = in && l >= g.F.k && l <= max_bases;
 	const unsigned m = __ballot_sync(kFull, mine);
 	if (mine) {
 		const int q = __popc(m & ((1u << lane) - 1u));
@@ -198,6 +268,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 	constexpr bool SCORE = WHAT != kLaneHits, HITS = WHAT != kLaneScores;
 	__shared__ LaneWarp<MODE> warps[kLaneWarps];
 	__shared__ LaneTables tab;
+	__shared__ LaneShare sh;
 	__shared__ double terms[MODE == SCORE_HARMONIC ? kHarmTerms : 1];
 	const ClassifyArgs &a = g.a;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -208,19 +279,33 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 		lane_tables<PACKED>(tab, g.F.k, lane);
 	if (MODE == SCORE_HARMONIC && threadIdx.x < kHarmTerms)
 		terms[threadIdx.x] = harmonic_term(threadIdx.x);
+	if (threadIdx.x == 32) {
+		const unsigned long long nmid = g.stats[kLaneMid];
+		const bool mids = lane_mids<SCORE>(g.F.keep != 0, nmid, a.n * a.mates);
+		sh.nlong = (uint32_t)g.stats[kLaneLong];
+		sh.listed = sh.nlong + (mids ? 0u : (uint32_t)nmid);
+		sh.max_bases = mids ? kLaneMaxBases : kLaneShortBases;
+		sh.own = sh.listed ? 0u : gridDim.x * kLaneWarps;
+		sh.warps = (uint32_t)min((uint64_t)kLaneWarps,
+				(g.chunks + gridDim.x - 1) / gridDim.x);
+		sh.help = sh.listed > 4u * g.chunks;
+		sh.go = !a.lane_stats || lane_has(a);
+	}
 	__syncthreads();
+	if (!sh.go)
+		return;
 
-	/* long reads, a warp each */
-	const unsigned long long nlong = *g.nlong;
-	if (nlong) {
+	/* listed reads, a warp each */
+	if (sh.listed && (warp < (int)sh.warps || sh.help)) {
 		for (;;) {
-			unsigned long long it = 0;
+			uint32_t it = 0;
 			if (lane == 0)
-				it = atomicAdd(g.ctr + 1, 1ull);
+				it = (uint32_t)atomicAdd(g.ctr + 1, 1ull);
 			it = __shfl_sync(kFull, it, 0);
-			if (it >= nlong)
+			if (it >= sh.listed)
 				break;
-			const uint32_t r = g.list[it];
+			const uint32_t r = g.list[it < sh.nlong ? it
+			                                        : (uint32_t)(a.n * a.mates) - 1u - (it - sh.nlong)];
 			const int d = lane_long_item<MODE, WHAT, COUNT, PACKED>(a, &g.sa, g.F, g.f, tab, r,
 					&w.nib[0][0], lane, COUNT ? acc : nullptr);
 			if (HITS && lane == 0)
@@ -232,7 +317,10 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 	/* the others, a lane each */
 	const int32_t k = (int32_t)g.F.k;
 	const uint64_t pol = lane_policy(g.F.keep != 0);
-	bool more = true;
+	if (lane == 0)
+		w.first = !sh.listed;
+	__syncwarp();
+	bool more = warp < (int)sh.warps;
 	int qi = 0, qn = 0;         /* queue: next item, items */
 	bool active = false;
 	bool open = false;          /* both: the decision has not fallen */
@@ -247,14 +335,17 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 				if (qi == qn) {
 					if (!more)
 						break;
-					unsigned long long c = 0;
-					if (lane == 0)
-						c = atomicAdd(g.ctr, 1ull);
+					unsigned long long c = (unsigned long long)warp * gridDim.x + blockIdx.x;
+					if (lane == 0) {
+						if (!w.first)
+							c = sh.own + atomicAdd(g.ctr, 1ull);
+						w.first = 0;
+					}
 					c = __shfl_sync(kFull, c, 0);
 					more = c < g.chunks;
 					if (!more)
 						break;
-					qn = lane_queue<MODE, WHAT, PACKED>(g, w, c, lane);
+					qn = lane_queue<MODE, WHAT, PACKED>(g, w, c, sh.max_bases, lane);
 					qi = 0;
 					if (!qn)
 						continue;
@@ -410,7 +501,7 @@ cudaError_t launch_mode(const LaneArgs &g, int num_sms, cudaStream_t s)
 				(228 << 10) - 1) / (228 << 10)));
 	if (e != cudaSuccess)
 		return e;
-	const uint64_t need = (g.chunks + kLaneWarps - 1) / kLaneWarps;
+	const uint64_t need = (g.a.n * g.a.mates + kLaneWarps - 1) / kLaneWarps;
 	const uint64_t full = (uint64_t)std::max(per_sm, 1) * num_sms;
 	kern<<<(unsigned)std::min(need, full), kLaneWarps * 32, 0, s>>>(g);
 	return cudaGetLastError();
@@ -439,38 +530,79 @@ bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64
 	return true;
 }
 
-/* Whether a filter of the call fits L2. */
-static bool lane_in_l2(const FilterDev *hf, uint32_t nf)
+/* Where the lane kernel is the faster one for every mixture of lengths, and where that
+ * depends on them.  A launch lasts as long as its longest read's lane (95 us for 150
+ * bases over a filter in L2, 154 over one in HBM, for any batch of up to some 28,000
+ * reads), the other kernels' time grows with the bases; ragged reads below are 50 to 300
+ * bases, log-uniform.
+ *
+ * - one filter in L2: from 20,000 reads on where these are short and of much the same
+ *   length (20,000 / 28,000 / 40,000 reads, 3.4 MB: 150 bases 95 / 93 / 106 us against
+ *   115 / 135 / 166, 300 bases 145 / 151 / 172 against 144 / 173 / 217, 600 bases 258 /
+ *   260 / 300 against 206 / 254 / 327, ragged 154 / 153 / 171 against 119 / 139 / 176),
+ *   from 40,000 on always; scores, every frame of which is walked, from 20,000 on always.
+ * - two to four that fit L2 together: the filter-major passes hash a read once for all of
+ *   them.  Four of 3.4 MB, 28,000 / 50,000 reads: 150 bases 270 / 326 us against 297 /
+ *   466, 600 bases 914 / 1110 against 946 / 1608; 28,000 / 100,000 ragged ones 501 / 874
+ *   against 334 / 805.  Scores of ragged reads 522 against 448 at 28,000, 571 against 577
+ *   at 40,000.
+ * - more that fit L2 together: likewise, and a launch's latency for each.  Ten of 3.4 MB
+ *   meet at 50,000 reads (150 bases 751 against 872, 300 bases 1423 against 1634), thirty
+ *   at 75,000 (80,000: 3007 against 3478); scores at 20,000 (150 bases 611 against 639) and
+ *   42,000 (50,000 of 50 bases: 816 against 1014).  100,000 ragged reads over ten 2149
+ *   against 1626, and one long read would make every launch wait.
+ * - filters that each fit L2 but not together: the passes miss L2 as well.  Ten of 68 MB,
+ *   from 28,000 reads on (50 bases 354 us against 400, 150 bases 852 against 1195, 1,000
+ *   bases 4765 against 7503; 20,000 of 50 bases 336 against 288), ragged ones from 60,000
+ *   (28,000 / 40,000: 1442 / 1575 against 1162 / 1404).  Scores of reads of which 5 % have
+ *   300 to 10,000 bases: 28,000 5204 us against 4976, 40,000 5378 against 5780.
+ * - one filter in HBM: a lane waits longer for its probes.  28,000 / 80,000 / 160,000 reads,
+ *   2.1 GB: 100 bases 116 / 216 / 331 us against 144 / 281 / 508, 150 bases 154 / 305 / 487
+ *   against 164 / 339 / 616, 300 bases 265 / 569 / 940 against 240 / 535 / 996; 40,000 /
+ *   60,000 ragged ones 248 / 305 against 205 / 275.  Scores: 100 bases 185 / 437 / 653
+ *   against 210 / 456 / 841, 150 bases 266 / 691 / 1053 against 286 / 655 / 1211, 300 bases
+ *   515 / 1437 / 2190 against 501 / 1234 / 2375.
+ * - several, one or more of them in HBM: the read-major kernel's probes of all filters
+ *   overlap.  3.4 MB and 2.1 GB, 28,000 / 40,000 ragged reads 334 / 383 us against 249 /
+ *   315, scores of 50,000 / 160,000 reads of 150 bases 543 / 1310 against 490 / 1406. */
+LaneRule lane_rule(const FilterDev *hf, uint32_t nf, bool scores, uint64_t reads)
 {
-	for (uint32_t i = 0; i < nf; ++i)
-		if (hf[i].m / 8 <= kLaneKeepBytes)
-			return true;
-	return false;
+	const uint64_t always = ~0ull;
+	const uint32_t none = ~0u, any = 0, free = ~0u;
+	uint64_t bytes = 0, most = 0;
+	for (uint32_t i = 0; i < nf; ++i) {
+		bytes += hf[i].m / 8;
+		most = std::max(most, hf[i].m / 8);
+	}
+	if (most > kLaneKeepBytes && nf > 1)
+		return {160000, always, 8, 8, free, false};
+	if (most > kLaneKeepBytes)
+		return {28000, 160000, 8, any, scores ? 130u : 170u, reads < 100000};
+	if (bytes > kLaneKeepBytes)
+		return {28000, 60000, any, scores && reads < 40000 ? 64 : any, free, true};
+	if (nf == 1)
+		return {20000, scores ? 20000u : 40000u, 8, any, reads < 28000 ? 170u : 250u, true};
+	if (nf <= 4)
+		return {20000, scores ? 40000u : 150000u, reads < 40000 ? 8 : any, any,
+				reads < 28000 ? 120u : free, true};
+	if (scores)
+		return {nf <= 10 ? 20000 : std::max<uint64_t>(28000, 1400ull * nf), always, 64, none, free,
+				true};
+	return {std::max<uint64_t>(std::min<uint64_t>(60000, 5000ull * nf), 2500ull * nf), always, 64,
+			none, free, true};
 }
 
-/* A lane's read takes its time (82 us for 150 bases over a filter in L2, 115-138 us
- * over one in HBM, the same for any batch of up to 37,888 reads); the other kernels'
- * time grows with the batch and reaches that at about 20k reads in L2 (82 us) and 28k
- * in HBM (122 us per 24k, 151 per 32k).  So it does with a few filters (four: 267
- * against 270 us at 20k) and with many that do not fit L2 together (ten of 68 MB: 927
- * against 836 at 20k).  Many that do fit are another matter: the filter-major passes
- * hash a read once for all of them and find them all in L2, the lane kernel pays a
- * launch's latency for each.  Ten of 3.4 MB meet at 50k reads (852 against 867 us;
- * 20k: 433 against 637), thirty at 60k (2584 against 2575; 20k: 954 against 1865).
- * Scores are walked per filter either way: ten meet at 20k (621 against 634), thirty
- * at 28k (1852 against 1857; 20k: 1410 against 1843). */
-bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads, bool scores)
+cudaError_t launch_lane_list(const ClassifyArgs &a, const LaneScratch &ls, int num_sms,
+		cudaStream_t s)
 {
-	if (!lane_in_l2(hf, nf))
-		return total_reads >= 28000;
-	uint64_t bytes = 0;
-	for (uint32_t i = 0; i < nf; ++i)
-		bytes += hf[i].m / 8;
-	if (nf <= 4 || bytes > kLaneKeepBytes)
-		return total_reads >= 20000;
-	if (scores)
-		return total_reads >= (nf <= 10 ? 20000u : 28000u);
-	return total_reads >= std::min<uint64_t>(60000, 5000ull * nf);
+	const uint64_t total = a.n * a.mates;
+	cudaError_t e = cudaMemsetAsync(ls.ctr, 0, kLaneStats * sizeof(unsigned long long), s);
+	if (e != cudaSuccess || total == 0)
+		return e;
+	const uint64_t need = (total + 255) / 256;
+	lane_list_kernel<<<(unsigned)std::min<uint64_t>(need, (uint64_t)num_sms * 8), 256, 0, s>>>(a,
+			ls.list, ls.ctr);
+	return cudaGetLastError();
 }
 
 cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreArgs *sa,
@@ -479,22 +611,16 @@ cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreA
 	const uint64_t total = a.n * a.mates;
 	if (total == 0)
 		return cudaSuccess;
-	cudaError_t e = cudaMemsetAsync(ls.ctr, 0, lane_counters(a.nf) * sizeof(unsigned long long), s);
-	if (e != cudaSuccess)
-		return e;
 	LaneArgs g;
-	g.max_bases = lane_in_l2(hf, a.nf) ? kLaneMaxBases : kLaneMaxBasesHbm;
-	const uint64_t need = (total + 255) / 256;
-	lane_long_kernel<<<(unsigned)std::min<uint64_t>(need, (uint64_t)num_sms * 8), 256, 0, s>>>(a,
-			g.max_bases, ls.list, ls.ctr);
-	if ((e = cudaGetLastError()) != cudaSuccess)
+	g.ctr = ls.ctr + kLaneStats;
+	cudaError_t e = cudaMemsetAsync(g.ctr, 0, 2 * (size_t)a.nf * sizeof(unsigned long long), s);
+	if (e != cudaSuccess)
 		return e;
 	g.a = a;
 	g.sa = sa ? *sa : ScoreArgs();
 	g.list = ls.list;
-	g.nlong = ls.ctr;
+	g.stats = ls.ctr;
 	g.chunks = (total + 31) / 32;
-	g.ctr = ls.ctr + 1;
 	for (g.f = 0; g.f < a.nf; ++g.f, g.ctr += 2) {
 		g.F = lane_filter(hf[g.f]);
 		e = sa ? (hits ? launch_lane_as<kLaneBoth, false>(g, num_sms, s)

@@ -22,28 +22,62 @@ namespace bbt {
  * one of 384 (8,000 over the small filter: 255 us, steps alone 659). */
 constexpr uint32_t kWindowBases = 1536;
 
-/* Device scratch of a launch: the indexes of the batch's long reads (n * mates
- * entries) and lane_counters(nf) counters, zeroed by the launch. */
+/* What lane_list_kernel finds of a batch's lengths: reads above kLaneMaxBases, reads
+ * above kLaneShortBases up to there, bases of the others and the longest of these. */
+enum { kLaneLong, kLaneMid, kLaneBases, kLaneLongest, kLaneStats };
+constexpr uint32_t kLaneMaxBases = 1024, kLaneShortBases = 384;
+
+/* Whether the lane kernel takes a batch of so many reads with these lengths.  Where
+ * one read in 64 is long the other kernels wait for the last of these (the lane kernel
+ * starts with them), whatever the short ones are. */
+__host__ __device__ inline bool lane_takes(const LaneRule &r, const unsigned long long *st,
+		uint64_t reads)
+{
+	if (st[kLaneMid] * r.mids > reads || st[kLaneLong] * r.longs > reads)
+		return false;
+	if (st[kLaneLong] * 64 >= reads)
+		return true;
+	const uint64_t shorts = reads - st[kLaneLong] - st[kLaneMid];
+	return st[kLaneBases] <= r.mean * shorts &&
+			(!r.even || 5 * st[kLaneBases] >= 4 * st[kLaneLongest] * shorts);
+}
+
+#if defined(__CUDACC__)
+/* A batch that is decided on the device: is it the lane kernel's? */
+__device__ __forceinline__ bool lane_has(const ClassifyArgs &a)
+{
+	return lane_takes(a.lane_rule, a.lane_stats, a.n * a.mates);
+}
+#endif
+
+/* Device scratch of a launch: the indexes of the batch's reads above kLaneShortBases
+ * (n * mates entries: those above kLaneMaxBases from the front, the others from the
+ * back) and lane_counters(nf) counters, of which the first kLaneStats are the
+ * counts. */
 struct LaneScratch {
 	uint32_t *list;
 	unsigned long long *ctr;
 };
 
-/* Whether the lane kernel takes these filters and options, and whether it is the
- * faster one for a batch of so many reads. */
+/* Whether the lane kernel can take these filters and options at all, and which
+ * batches it is the faster one for. */
 bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64_t total_reads);
-bool lane_pays(const FilterDev *hf, uint32_t nf, uint64_t total_reads, bool scores);
+LaneRule lane_rule(const FilterDev *hf, uint32_t nf, bool scores, uint64_t reads);
 
-/* Counters of a launch (which is a kernel per filter, after one that lists long
- * reads). */
+/* Counters of a launch (which is a kernel per filter, after one that lists the
+ * longer reads). */
 inline size_t lane_counters(uint32_t nf)
 {
-	return 1 + 2 * (size_t)nf;
+	return kLaneStats + 2 * (size_t)nf;
 }
 
-/* Hits of a batch (sa NULL), or the scores of every (read, filter) into
- * sa->scores, and with `hits` both in one walk (count: hits alone).  With two or more filters the hit words are ORed into and must be
- * zeroed before. */
+/* The list and the counts, which every launch_lane over the batch reads. */
+cudaError_t launch_lane_list(const ClassifyArgs &a, const LaneScratch &ls, int num_sms,
+		cudaStream_t s);
+
+/* Hits of a batch (sa NULL), or the scores of every (read, filter) into sa->scores,
+ * and with `hits` both in one walk (count: hits alone).  With two or more filters the
+ * hit words are ORed into and must be zeroed before. */
 cudaError_t launch_lane(const ClassifyArgs &a, const FilterDev *hf, const ScoreArgs *sa,
 		bool hits, const LaneScratch &ls, int num_sms, bool count, cudaStream_t s);
 

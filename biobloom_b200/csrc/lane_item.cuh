@@ -8,17 +8,13 @@
 
 #include "bbt.h"
 #include "classify.cuh"
+#include "lane.cuh"
 #include "lane_walk.cuh"
 #include "score_value.cuh"
 #include "window.cuh"
 
 namespace bbt {
 
-/* Reads above this many bases are evaluated by whole warps: a lane's steps take
- * one after another the latency of h probes each, which is longer for a filter
- * in HBM (2.1 GB filter, 50k reads of 50 bp to 10 kb: 489 us at 384, 505 at 512,
- * 610 at 1024); over a filter in L2 a lane costs half the instructions. */
-constexpr uint32_t kLaneMaxBases = 1024, kLaneMaxBasesHbm = 384;
 constexpr uint64_t kLaneKeepBytes = 126ull << 20; /* L2 */
 
 /* A filter as the lane kernel probes it (m = 32 m5 bits). */

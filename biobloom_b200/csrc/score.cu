@@ -16,6 +16,7 @@
  * its hit bits come from the classification kernel.
  */
 #include "classify.cuh"
+#include "lane.cuh"
 #include "score_value.cuh"
 #include "seqeval_chunk.cuh"
 #include "window.cuh"
@@ -100,6 +101,8 @@ template <int SEG, int MODE>
 __global__ void __launch_bounds__(256, 4) score_kernel(ClassifyArgs a, ScoreArgs sa)
 {
 	extern __shared__ __align__(16) unsigned char smem[];
+	if (a.lane_stats && lane_has(a))
+		return;
 	const int lane = threadIdx.x & 31;
 	const int warp = threadIdx.x >> 5;
 	const Window<SEG> win = window_at<SEG>(smem + warp * window_stride<SEG>(a.kmax));
@@ -133,6 +136,8 @@ cudaError_t launch_score_seg(const ClassifyArgs &a, const ScoreArgs &sa, const L
 /* evaluateReadBestHit over stored scores: one thread per read (mate). */
 __global__ void best_hits_kernel(ClassifyArgs a, const double *s0, const double *s1)
 {
+	if (a.lane_stats && !lane_has(a))
+		return; /* the scores are the other kernel's, which writes the hits itself */
 	const uint64_t total = a.n * a.mates;
 	for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < total;
 			r += (uint64_t)gridDim.x * blockDim.x) {
