@@ -224,8 +224,9 @@ extern "C" int bbt_close(bbt_ctx *ctx)
 	}
 	if (ctx->ev_start)
 		cudaEventDestroy(ctx->ev_start);
-	if (ctx->ev_stop)
-		cudaEventDestroy(ctx->ev_stop);
+	for (cudaEvent_t e : ctx->ev_stop)
+		if (e)
+			cudaEventDestroy(e);
 	if (ctx->ev_k0)
 		cudaEventDestroy(ctx->ev_k0);
 	if (ctx->ev_k1)
@@ -475,7 +476,8 @@ extern "C" int bbt_open(const char *const *bf_paths, int n_filters, const bbt_pa
 	OPEN_TRY(cudaStreamCreateWithFlags(&ctx->h2d, cudaStreamNonBlocking));
 	OPEN_TRY(cudaStreamCreateWithFlags(&ctx->d2h, cudaStreamNonBlocking));
 	OPEN_TRY(cudaEventCreate(&ctx->ev_start));
-	OPEN_TRY(cudaEventCreate(&ctx->ev_stop));
+	for (cudaEvent_t &e : ctx->ev_stop)
+		OPEN_TRY(cudaEventCreate(&e));
 	OPEN_TRY(cudaEventCreate(&ctx->ev_k0));
 	OPEN_TRY(cudaEventCreate(&ctx->ev_k1));
 	for (Slot &s : ctx->slot) {
@@ -780,6 +782,36 @@ static bool grow_if_room(T **buf, uint64_t &cap, uint64_t n)
 	return true;
 }
 
+/* Before a call's first use of the context's scratch, on stream s: after the call that
+ * used it last, if that was on another stream.  (A captured graph has its own; one that
+ * the caller captures cannot wait for what runs outside it.) */
+static int claim_scratch(bbt_ctx *ctx, cudaStream_t s)
+{
+	if (ctx->capturing || ctx->callers_capture || ctx->claimed)
+		return BBT_OK;
+	unsigned long long id = 0; /* unlike its address, never another stream's */
+	CUDA_TRY(ctx, cudaStreamGetId(s, &id));
+	if (id != ctx->scratch_stream)
+		CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_stop[1], 0));
+	ctx->scratch_stream = id;
+	ctx->claimed = true;
+	return BBT_OK;
+}
+
+/* A point of a call's timeline; none in a graph, whose replays are not timed. */
+static cudaError_t mark(const bbt_ctx *ctx, cudaEvent_t e, cudaStream_t s)
+{
+	return ctx->capturing || ctx->callers_capture ? cudaSuccess : cudaEventRecord(e, s);
+}
+
+/* The end of a call, and of its use of the scratch. */
+static cudaError_t mark_stop(bbt_ctx *ctx, cudaStream_t s)
+{
+	ctx->last_stop = ctx->claimed;
+	ctx->claimed = false;
+	return mark(ctx, ctx->ev_stop[ctx->last_stop], s);
+}
+
 /* Two-pass filter-major classification of one batch (all filters share k):
  * scan of padded frame counts, a host read of the per-block totals to cut the
  * batch into sub-batches whose frames fit the scratch, then hash pass and
@@ -791,7 +823,9 @@ static int run_two_pass(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s,
 	const uint64_t B = two_pass_block_reads();
 	const uint64_t nb = (total + B - 1) / B;
 	const unsigned k = ctx->hf[0].k;
-	int rc = grow(ctx, &ctx->d_tp_local, ctx->tp_local_cap, total);
+	int rc = claim_scratch(ctx, s);
+	if (!rc)
+		rc = grow(ctx, &ctx->d_tp_local, ctx->tp_local_cap, total);
 	if (rc)
 		return rc;
 	if (nb + 1 > ctx->tp_sums_cap) {
@@ -1004,6 +1038,9 @@ static int run_bucketed(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s)
 {
 	const uint64_t total = a.n * a.mates;
 	const size_t hb = a.n * ctx->words * sizeof(uint64_t);
+	int rc = claim_scratch(ctx, s);
+	if (rc)
+		return rc;
 	CUDA_TRY(ctx, cudaMemsetAsync(a.hits[0], 0, hb, s));
 	if (a.mates == 2)
 		CUDA_TRY(ctx, cudaMemsetAsync(a.hits[1], 0, hb, s));
@@ -1023,7 +1060,7 @@ static int run_bucketed(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s)
 	size_t scan_bytes = 0;
 	CUDA_TRY(ctx, cub::DeviceScan::InclusiveSum(nullptr, scan_bytes, ctx->d_bk_fo + 1,
 			ctx->d_bk_fo + 1, total, s));
-	int rc = bk_tmp(ctx, scan_bytes);
+	rc = bk_tmp(ctx, scan_bytes);
 	if (rc)
 		return rc;
 	const uint32_t levels = std::max<uint32_t>(ctx->bk_levels, 1);
@@ -1179,9 +1216,12 @@ static int run_dust(bbt_ctx *ctx, ClassifyArgs &a, const uint64_t *mate_bases, c
 {
 	DustArgs d;
 	memset(&d, 0, sizeof d);
+	int rc = claim_scratch(ctx, s);
+	if (rc)
+		return rc;
 	for (uint32_t m = 0; m < a.mates; ++m) {
 		const uint64_t words = mate_bases[m] / 32 + 2;
-		int rc = grow(ctx, &ctx->d_dust[m], ctx->dust_words_cap[m], words);
+		rc = grow(ctx, &ctx->d_dust[m], ctx->dust_words_cap[m], words);
 		if (rc)
 			return rc;
 		CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_dust[m], 0, words * sizeof(uint32_t), s));
@@ -1190,7 +1230,7 @@ static int run_dust(bbt_ctx *ctx, ClassifyArgs &a, const uint64_t *mate_bases, c
 		d.off_base[m] = a.off_base[m];
 		d.mask[m] = ctx->d_dust[m];
 	}
-	int rc = grow(ctx, &ctx->d_dust_redo, ctx->dust_redo_cap, 2 * a.n * a.mates);
+	rc = grow(ctx, &ctx->d_dust_redo, ctx->dust_redo_cap, 2 * a.n * a.mates);
 	if (rc)
 		return rc;
 	CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_dust_cnt, 0, sizeof(unsigned long long), s));
@@ -1293,10 +1333,13 @@ static int run_warps(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreA
 		LaunchConfig lc = ctx->lc;
 		if (lc.path == BBT_PATH_FILTER_MAJOR)
 			lc.path = BBT_PATH_PERSISTENT; /* filters of different k */
+		int rc = lc.path != BBT_PATH_PLAIN ? claim_scratch(ctx, s) : BBT_OK;
+		if (rc)
+			return rc;
 		if (lc.path != BBT_PATH_PLAIN)
 			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.work, 0, sizeof(unsigned long long), s));
 		if (lc.path != BBT_PATH_PLAIN && ctx->long_bases) {
-			int rc = grow(ctx, &ctx->sc.order, ctx->sc.order_cap, a.n * a.mates);
+			rc = grow(ctx, &ctx->sc.order, ctx->sc.order_cap, a.n * a.mates);
 			if (rc)
 				return rc;
 			CUDA_TRY(ctx, cudaMemsetAsync(ctx->sc.order_cnt, 0,
@@ -1358,12 +1401,17 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	if (lane && ctx->capturing && (a.n * a.mates > ctx->sc.lane_list_cap ||
 			(best_only && a.n * ctx->nf > ctx->sc.scores_cap)))
 		lane = kLaneNo;
-	if (lane) {
-		int rc = grow(ctx, &ctx->sc.lane_list, ctx->sc.lane_list_cap, a.n * a.mates);
+	/* a graph that the caller captures must not hold buffers that a later call replaces */
+	if (ctx->callers_capture)
+		lane = kLaneNo;
+	if (lane || (best_only && two_pass)) {
+		int rc = claim_scratch(ctx, s);
+		if (!rc && lane)
+			rc = grow(ctx, &ctx->sc.lane_list, ctx->sc.lane_list_cap, a.n * a.mates);
 		if (rc)
 			return rc;
 	}
-	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_k0, s));
+	CUDA_TRY(ctx, mark(ctx, ctx->ev_k0, s));
 	if (lane) {
 		const LaneScratch ls = lane_scratch(ctx->sc);
 		CUDA_TRY(ctx, launch_lane_list(a, ls, ctx->num_sms, s));
@@ -1416,7 +1464,7 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	}
 	if (rc)
 		return rc;
-	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_k1, s));
+	CUDA_TRY(ctx, mark(ctx, ctx->ev_k1, s));
 	CUDA_TRY(ctx, launch_summarize(a.hits[0], a.mates == 2 ? a.hits[1] : nullptr, a.n, ctx->nf,
 			ctx->words, ctx->p.inclusive, ctx->mode == BBT_MODE_ORDERED, d_cat, ctx->d_counts,
 			ctx->num_sms, s));
@@ -1437,8 +1485,8 @@ static int ensure_tmp_hits(bbt_ctx *ctx, uint64_t n)
 	return BBT_OK;
 }
 
-static int classify_device(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cudaStream_t s,
-		double *const *scores = nullptr)
+static int classify_device_batch(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cudaStream_t s,
+		double *const *scores)
 {
 	const bool paired = b->seq2 != nullptr;
 	if (ctx->p.scoring == BBT_SCORE_BINOMIAL && ctx->mode != BBT_MODE_BESTHIT &&
@@ -1465,7 +1513,9 @@ static int classify_device(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cuda
 	a.n = b->n_reads;
 	a.mates = paired ? 2 : 1;
 	if (!r->hits || (paired && !r->hits2)) {
-		int rc = ensure_tmp_hits(ctx, b->n_reads);
+		int rc = claim_scratch(ctx, s);
+		if (!rc)
+			rc = ensure_tmp_hits(ctx, b->n_reads);
 		if (rc)
 			return rc;
 	}
@@ -1487,13 +1537,16 @@ static int classify_device(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cuda
 			mate_bases[m] = ends[1] - ends[0];
 			a.seq[m] += ends[0]; /* bases indexed from offsets[0] */
 		}
+		int rc = claim_scratch(ctx, s);
+		if (rc)
+			return rc;
 		CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_dust_cnt + 1, 0, sizeof(unsigned long long), s));
 	}
-	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, s));
+	CUDA_TRY(ctx, mark(ctx, ctx->ev_start, s));
 	int rc = run_kernels(ctx, a, r->category, s, scores, mate_bases);
 	if (rc)
 		return rc;
-	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, s));
+	CUDA_TRY(ctx, mark_stop(ctx, s));
 	if (ctx->dust) {
 		CUDA_TRY(ctx, cudaStreamSynchronize(s));
 		rc = dust_check(ctx);
@@ -1505,11 +1558,24 @@ static int classify_device(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cuda
 	return BBT_OK;
 }
 
+static int classify_device(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cudaStream_t s,
+		double *const *scores = nullptr)
+{
+	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+	CUDA_TRY(ctx, cudaStreamIsCapturing(s, &st));
+	ctx->callers_capture = !ctx->capturing && st != cudaStreamCaptureStatusNone;
+	const int rc = classify_device_batch(ctx, b, r, s, scores);
+	ctx->callers_capture = false;
+	if (ctx->claimed) /* it failed on the way: what it launched still uses the scratch */
+		mark_stop(ctx, s);
+	return rc;
+}
+
 /* Host batches: split into sub-batches that fit the staging slots; copies in
  * (h2d stream), kernels (ctx->stream) and copies out (d2h stream) of
  * consecutive sub-batches overlap, two slots deep. */
-static int classify_host(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r,
-		double *const *scores = nullptr)
+static int classify_host_batch(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r,
+		double *const *scores)
 {
 	const bool paired = b->seq2 != nullptr;
 	const uint64_t n = b->n_reads;
@@ -1573,10 +1639,14 @@ static int classify_host(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r,
 			r->category && host_pinned(r->category),
 			want_scores && scores[0] && host_pinned(scores[0]),
 			want_scores && paired && scores[1] && host_pinned(scores[1])};
-	if (ctx->dust)
+	if (ctx->dust) {
+		int rc = claim_scratch(ctx, ctx->stream);
+		if (rc)
+			return rc;
 		CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_dust_cnt + 1, 0, sizeof(unsigned long long),
 				ctx->stream));
-	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_start, ctx->stream));
+	}
+	CUDA_TRY(ctx, mark(ctx, ctx->ev_start, ctx->stream));
 	while (i0 < n) {
 		/* largest i1 with bases and reads inside the slot capacity */
 		uint64_t i1 = std::min(n, i0 + step);
@@ -1726,7 +1796,7 @@ static int classify_host(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r,
 		which ^= 1;
 		i0 = i1;
 	}
-	CUDA_TRY(ctx, cudaEventRecord(ctx->ev_stop, ctx->stream));
+	CUDA_TRY(ctx, mark_stop(ctx, ctx->stream));
 	CUDA_TRY(ctx, cudaStreamSynchronize(ctx->d2h));
 	CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
 	for (Slot &s : ctx->slot) {
@@ -1741,6 +1811,15 @@ static int classify_host(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r,
 	ctx->reads_seen += n;
 	ctx->last.reads = n * (paired ? 2 : 1);
 	return BBT_OK;
+}
+
+static int classify_host(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r,
+		double *const *scores = nullptr)
+{
+	const int rc = classify_host_batch(ctx, b, r, scores);
+	if (ctx->claimed)
+		mark_stop(ctx, ctx->stream);
+	return rc;
 }
 
 /* A host batch over this context's devices: contiguous shards of reads in
@@ -1994,9 +2073,10 @@ extern "C" int bbt_last_stats(bbt_ctx *ctx, bbt_stats *out)
 	if (!ctx || !out)
 		return BBT_ERR_ARG;
 	CUDA_TRY(ctx, cudaSetDevice(ctx->dev));
-	CUDA_TRY(ctx, cudaEventSynchronize(ctx->ev_stop));
+	const cudaEvent_t stop = ctx->ev_stop[ctx->last_stop];
+	CUDA_TRY(ctx, cudaEventSynchronize(stop));
 	float ms = 0, kms = 0;
-	CUDA_TRY(ctx, cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop));
+	CUDA_TRY(ctx, cudaEventElapsedTime(&ms, ctx->ev_start, stop));
 	CUDA_TRY(ctx, cudaEventElapsedTime(&kms, ctx->ev_k0, ctx->ev_k1));
 	ctx->last.kernel_ms = ms;
 	ctx->last.classify_ms = kms;

@@ -130,7 +130,8 @@ struct bbt_ctx {
 	std::shared_ptr<uint32_t> bthres; /* on the device; a captured graph keeps the one it reads */
 	uint64_t bt_rows = 0;
 	unsigned int *d_lenset = nullptr;
-	bool capturing = false;          /* a CUDA graph is being captured */
+	bool capturing = false;          /* a CUDA graph is being captured, with scratch of its own */
+	bool callers_capture = false;    /* this call's stream is being captured by the caller */
 	/* -d / -n: print reads of the first filter (or all others) to stdout */
 	bool to_stdout = false, inverse = false;
 	/* long-first read order of the persistent kernel (0 = index order) */
@@ -170,7 +171,13 @@ struct bbt_ctx {
 	/* bbt_open_devices: the same filters opened on the other devices; host
 	 * batches are split across this context and these */
 	std::vector<bbt_ctx *> peers;
-	cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
+	/* ev_stop[1]: the end of the last call that used the context's scratch (sc, d_tmp_*
+	 * and the buffers of masking and of the two-pass and bucketed paths), which calls on
+	 * other streams wait for before they use it; [0]: of the last call that did not */
+	cudaEvent_t ev_start = nullptr, ev_stop[2] = {nullptr, nullptr};
+	int last_stop = 0;                     /* of the last call */
+	bool claimed = false;                  /* this call uses the scratch */
+	unsigned long long scratch_stream = 0; /* ID of the stream that used it last */
 	cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr; /* around the last classify kernel */
 	bbt::LaunchConfig lc;
 	bbt_stats last = {0, 0, 0, 0, 0.0, 0.0, 0};

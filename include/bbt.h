@@ -183,7 +183,9 @@ typedef struct {
  * copies overlapping the kernels of the one before; pinned host arrays
  * overlap best, results bound for pageable memory are staged through pinned
  * buffers); with BBT_DEVICE buffers it enqueues on `stream` and returns
- * (results are ready when the stream reaches that point).
+ * (results are ready when the stream reaches that point).  Calls of one context on
+ * several streams may be in flight together: where they use its scratch buffers, a
+ * call's kernels wait for those of the call before on another stream.
  */
 int bbt_classify_batch(bbt_ctx *ctx, const bbt_batch *batch, bbt_result *result,
 		void *stream);
