@@ -408,16 +408,12 @@ cudaError_t launch_one(const ClassifyArgs &a, const LaunchConfig &lc, cudaStream
 	          : a.scoring == BBT_SCORE_HARMONIC ? classify_kernel<SEG, ORDER, C, BBT_SCORE_HARMONIC, WIDE>
 	          : a.scoring == BBT_SCORE_BINOMIAL ? classify_kernel<SEG, ORDER, C, BBT_SCORE_BINOMIAL, WIDE>
 	                                            : classify_kernel<SEG, ORDER, C, BBT_SCORE_SIMPLE, WIDE>;
-	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			(int)smem);
-	if (e != cudaSuccess)
-		return e;
 	uint64_t total = a.n * a.mates;
 	uint64_t warps_needed = total;
 	unsigned blocks;
 	if (ORDER != ORDER_PLAIN) {
 		int per_sm = 0;
-		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
+		cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem);
 		if (e != cudaSuccess)
 			return e;
 		if (per_sm < 1)
@@ -454,6 +450,9 @@ cudaError_t launch_seg(const ClassifyArgs &a, const LaunchConfig &lc, cudaStream
 
 } // namespace
 
+/* At most 8 warps' windows, 27 KB: below what a launch may have without raising its
+ * kernel's limit, which belongs to the process (a thread with a smaller k would lower
+ * it between another's setting and its launch). */
 size_t classify_smem_bytes(const LaunchConfig &lc, uint32_t kmax)
 {
 	const size_t per_warp = lc.seg == 8 ? window_stride<8>(kmax) : window_stride<4>(kmax);

@@ -1208,13 +1208,25 @@ static cudaError_t launch_h(const MibfArgs &a, int grid, size_t smem, cudaStream
 	return cudaGetLastError();
 }
 
+/* Raises a kernel's limit of dynamic shared memory as far as it goes, not to what one
+ * launch takes: the limit belongs to the process, where another thread's context may
+ * take more. */
+template <class K>
+static cudaError_t raise_smem(K kern)
+{
+	cudaFuncAttributes at;
+	const cudaError_t e = cudaFuncGetAttributes(&at, kern);
+	return e != cudaSuccess ? e : cudaFuncSetAttribute(kern,
+			cudaFuncAttributeMaxDynamicSharedMemorySize, (227 << 10) - (int)at.sharedSizeBytes);
+}
+
 /* Blocks per SM of a variant with smem bytes of shared memory (also sets the
  * variant's shared-memory limit, which must precede its launch). */
 template <int H, bool D, bool B, bool P = false>
 static int occupancy_h(size_t smem)
 {
 	auto kern = mibf_query_kernel<H, D, Fpl<H, D>::value, B, P>;
-	cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	raise_smem(kern);
 	int nb = 0;
 	cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kQueryThreads, smem);
 	return nb > 0 ? nb : 1;
@@ -1729,8 +1741,7 @@ static int mbk_grow(bbt_mibf *ctx, T **p, uint64_t &cap, uint64_t n)
 template <int H>
 static cudaError_t mbk_launch_hash(const MbkArgs &b, size_t smem, cudaStream_t s)
 {
-	cudaError_t e = cudaFuncSetAttribute(mbk_hash_kernel<H>,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+	const cudaError_t e = raise_smem(mbk_hash_kernel<H>);
 	if (e != cudaSuccess)
 		return e;
 	mbk_hash_kernel<H><<<b.nblk, kMbkThreads, smem, s>>>(b);
@@ -1945,10 +1956,7 @@ template <int H>
 static cudaError_t launch_scan_h(const MibfArgs &a, const ScanLists &l, int num_sms, cudaStream_t s)
 {
 	const size_t smem = scan_smem(a.f.nids);
-	/* the limit of the most IDs, not of these: it belongs to the process, where
-	 * another thread's context may have more */
-	cudaError_t e = cudaFuncSetAttribute(mibf_scan_kernel<H>,
-			cudaFuncAttributeMaxDynamicSharedMemorySize, (int)scan_smem(kMibfSmemIds));
+	cudaError_t e = raise_smem(mibf_scan_kernel<H>);
 	int nb = 0;
 	if (e == cudaSuccess)
 		e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, mibf_scan_kernel<H>, kScanThreads,

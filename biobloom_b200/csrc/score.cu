@@ -121,10 +121,6 @@ cudaError_t launch_score_seg(const ClassifyArgs &a, const ScoreArgs &sa, const L
 	          : a.scoring == BBT_SCORE_HARMONIC ? score_kernel<SEG, SCORE_HARMONIC>
 	          : a.scoring == BBT_SCORE_BINOMIAL ? score_kernel<SEG, SCORE_BINOMIAL>
 	                                            : score_kernel<SEG, SCORE_SIMPLE>;
-	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-			(int)smem);
-	if (e != cudaSuccess)
-		return e;
 	const uint64_t total = a.n * a.mates;
 	const uint64_t blocks = (total + lc.warps_per_block - 1) / lc.warps_per_block;
 	if (blocks == 0)

@@ -460,9 +460,6 @@ cudaError_t two_pass_sub_batch(const ClassifyArgs &a, const TwoPassArgs &p, cons
 				(threads / 32);
 		auto kern = lc.seg == 8 ? (C ? hash_pass_kernel<8, true> : hash_pass_kernel<8, false>)
 		                        : (C ? hash_pass_kernel<4, true> : hash_pass_kernel<4, false>);
-		if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-				(int)smem)) != cudaSuccess)
-			return e;
 		kern<<<persistent_blocks(kern, threads, smem, lc.num_sms, nreads), threads, smem, s>>>(a, p);
 		if ((e = cudaGetLastError()) != cudaSuccess)
 			return e;

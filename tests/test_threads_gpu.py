@@ -62,20 +62,51 @@ def test_masking_windows(tmp_path):
         c.close()
 
 
-def test_numbers_of_ids(tmp_path):
+def test_window_sizes(tmp_path):
+    """k and the frames a lane hashes size the windows of the read-major and filter-major kernels."""
+    import torch
+    rng = np.random.default_rng(5)
+    opened, streams, got = [], [], {}
+    for k, frames, path in ((8, 4, 2), (60, 8, 2), (25, 8, 2), (8, 4, 3), (60, 8, 3)):
+        d = tmp_path / f"k{k}_{frames}_{path}"
+        d.mkdir()
+        genomes, filters, paths = _filters(d, rng, [k, k], 3)
+        reads = [r[:200] for r in _reads(rng, genomes, 120, k)]
+        c = _open(paths, ol.SIMPLE, 0.15, 3, path=path)
+        c.set_launch(path, 8, frames)
+        opened.append((c, _device(reads), ol.classify(*ol.pack_reads(reads), filters, 0.15, 3)[0]))
+        streams.append(torch.cuda.Stream())
+    torch.cuda.synchronize()
+
+    def call(i):
+        with torch.cuda.stream(streams[i]):
+            got[i] = opened[i][0].classify_device(*opened[i][1])[0]
+
+    raised = _at_once([lambda i=i: call(i) for i in range(len(opened))], 300)
+    assert not raised
+    torch.cuda.synchronize()
+    for i, (c, _, want) in enumerate(opened):
+        assert np.array_equal(got[i].cpu().numpy().view(np.uint64), want)
+        c.close()
+
+
+@pytest.mark.parametrize("long_read", [False, True])
+def test_numbers_of_ids(tmp_path, long_read):
+    """The scan kernel, and the general one, which a batch with a long read takes."""
     import torch
     from biobloom_b200.mibf import MIBFClassifier
     rng = np.random.default_rng(4)
     opened = []
     for n in (5, 400, 1000):
         targets = [_genome(rng, 200).tobytes() for _ in range(n)]
-        f = ol.MIBF.build(targets, list(range(1, n + 1)), k=25, h=3, occupancy=0.5)
+        f = ol.MIBF.build(targets, list(range(1, n + 1)), k=25, h=8, occupancy=0.5)
         f.store(str(tmp_path / f"x{n}"))
         with open(tmp_path / f"x{n}_ids.txt", "w") as fh:
             for i in range(n):
                 fh.write(f"{i + 1}\tt{i}\n")
         opened.append((MIBFClassifier(str(tmp_path / f"x{n}.bf"), layout=2),
-                       _device(targets[:5] * 20), torch.cuda.Stream()))
+                       _device(targets[:5] * 20 + [_genome(rng, 9000 if long_read else 90).tobytes()]),
+                       torch.cuda.Stream()))
     torch.cuda.synchronize()
     got = {}
 
@@ -89,6 +120,6 @@ def test_numbers_of_ids(tmp_path):
     torch.cuda.synchronize()
     for i, (c, _, _) in enumerate(opened):
         hits, n_hits, _ = (t.cpu().numpy() for t in got[i])
-        assert (n_hits == 1).all()
-        assert np.array_equal(hits.reshape(100, 2, -1)[:, 0, 0], np.tile(np.arange(1, 6), 20))
+        assert (n_hits[:100] == 1).all() and n_hits[100] == 0
+        assert np.array_equal(hits[:100, 0, 0], np.tile(np.arange(1, 6), 20))
         c.close()
