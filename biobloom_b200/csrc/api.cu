@@ -1399,17 +1399,22 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 		lane = kLaneNo;
 	/* no allocation while a graph is captured: with the scratch that it has */
 	if (lane && ctx->capturing && (a.n * a.mates > ctx->sc.lane_list_cap ||
-			(best_only && a.n * ctx->nf > ctx->sc.scores_cap)))
+			(best_only && a.n * a.mates * ctx->nf > ctx->sc.scores_cap)))
 		lane = kLaneNo;
 	/* a graph that the caller captures must not hold buffers that a later call replaces */
 	if (ctx->callers_capture)
 		lane = kLaneNo;
 	if (lane || (best_only && two_pass)) {
 		int rc = claim_scratch(ctx, s);
-		if (!rc && lane)
-			rc = grow(ctx, &ctx->sc.lane_list, ctx->sc.lane_list_cap, a.n * a.mates);
+		const uint64_t need = best_only ? a.n * a.mates * ctx->nf : 0;
+		if (!rc && two_pass)
+			rc = grow(ctx, &ctx->sc.scores, ctx->sc.scores_cap, need);
 		if (rc)
 			return rc;
+		/* without room for what the lane kernel takes, the kernels that need none */
+		if (!grow_if_room(&ctx->sc.scores, ctx->sc.scores_cap, need) ||
+				(lane && !grow_if_room(&ctx->sc.lane_list, ctx->sc.lane_list_cap, a.n * a.mates)))
+			lane = kLaneNo;
 	}
 	CUDA_TRY(ctx, mark(ctx, ctx->ev_k0, s));
 	if (lane) {
@@ -1430,18 +1435,8 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	/* the scores that BESTHIT's hits come from, where nobody asked for them */
 	ScoreArgs ps = sa;
 	if (best_only && (lane || two_pass)) {
-		const uint64_t need = a.n * ctx->nf;
-		if (need > ctx->sc.scores_cap) {
-			cudaFree(ctx->sc.scores[0]);
-			cudaFree(ctx->sc.scores[1]);
-			ctx->sc.scores[0] = ctx->sc.scores[1] = nullptr;
-			ctx->sc.scores_cap = 0;
-			CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[0], need * sizeof(double)));
-			CUDA_TRY(ctx, cudaMalloc(&ctx->sc.scores[1], need * sizeof(double)));
-			ctx->sc.scores_cap = need;
-		}
-		ps.scores[0] = ctx->sc.scores[0];
-		ps.scores[1] = a.mates == 2 ? ctx->sc.scores[1] : nullptr;
+		ps.scores[0] = ctx->sc.scores;
+		ps.scores[1] = a.mates == 2 ? ctx->sc.scores + a.n * ctx->nf : nullptr;
 	}
 	const bool stored = best || want_scores; /* scores go to memory (lane, two-pass) */
 	int rc = BBT_OK;
@@ -2406,12 +2401,8 @@ static int graph_scratch(bbt_ctx *ctx, BfScratch &sc, uint64_t reads, uint32_t m
 	LaneRule rule;
 	if (lane_use(ctx, ctx->lc, reads * mates, rule) &&
 			grow_if_room(&sc.lane_list, sc.lane_list_cap, reads * mates) &&
-			ctx->mode == BBT_MODE_BESTHIT && lane_stores_scores(ctx, reads, mates)) {
-		uint64_t cap[2] = {0, 0};
-		for (uint32_t m = 0; m < mates; ++m)
-			grow_if_room(&sc.scores[m], cap[m], reads * ctx->nf);
-		sc.scores_cap = cap[0] && (mates == 1 || cap[1]) ? reads * ctx->nf : 0;
-	}
+			ctx->mode == BBT_MODE_BESTHIT && lane_stores_scores(ctx, reads, mates))
+		grow_if_room(&sc.scores, sc.scores_cap, reads * mates * ctx->nf);
 	return BBT_OK;
 }
 
@@ -2543,8 +2534,7 @@ void bbt::bf_scratch_free(BfScratch &sc)
 	cudaFree(sc.order_cnt);
 	cudaFree(sc.order);
 	cudaFree(sc.lane_list);
-	cudaFree(sc.scores[0]);
-	cudaFree(sc.scores[1]);
+	cudaFree(sc.scores);
 	sc = BfScratch();
 }
 

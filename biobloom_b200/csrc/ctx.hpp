@@ -67,8 +67,9 @@ struct BfScratch {
 	uint64_t order_cap = 0;
 	uint32_t *lane_list = nullptr;           /* lane kernel (lane.cu): the batch's long reads */
 	uint64_t lane_list_cap = 0;
-	double *scores[2] = {nullptr, nullptr};  /* BESTHIT scores nobody asked for */
-	uint64_t scores_cap = 0;                 /* elements per mate array */
+	double *scores = nullptr;                /* BESTHIT scores nobody asked for: a mate array
+	                                            after the other */
+	uint64_t scores_cap = 0;                 /* elements */
 };
 
 } // namespace bbt
