@@ -1493,6 +1493,8 @@ extern "C" int bbt_mibf_close(bbt_mibf *ctx)
 			cudaEventDestroy(ctx->ev0);
 		if (ctx->ev1)
 			cudaEventDestroy(ctx->ev1);
+		if (ctx->ev_free)
+			cudaEventDestroy(ctx->ev_free);
 		if (ctx->stream)
 			cudaStreamDestroy(ctx->stream);
 	}
@@ -1535,7 +1537,8 @@ extern "C" int bbt_mibf_open(const char *bf_path, const bbt_mibf_params *params,
 	if (rc)
 		return bail(rc);
 	if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-			cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess)
+			cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
+			cudaEventCreateWithFlags(&ctx->ev_free, cudaEventDisableTiming) != cudaSuccess)
 		return bail(mibf_fail(ctx, BBT_ERR_CUDA, "cannot create a stream"));
 	rc = load_device(ctx, mibf_sdsl_path(bf_path), ids);
 	if (rc)
@@ -1614,7 +1617,7 @@ static int ensure_min_count(bbt_mibf *ctx, const std::vector<uint32_t> &fcs, cud
 		rows = std::max<uint32_t>(rows, 256);
 		uint32_t *d = nullptr;
 		MIBF_TRY(ctx, cudaMalloc(&d, (size_t)rows * nids * 4));
-		MIBF_TRY(ctx, cudaStreamSynchronize(s));
+		MIBF_TRY(ctx, cudaDeviceSynchronize()); /* no kernel may still read the old rows */
 		cudaFree(ctx->d_minc);
 		ctx->d_minc = d;
 		ctx->minc_rows = rows;
@@ -2058,6 +2061,13 @@ static int run_query_sc(bbt_mibf *ctx, uint64_t n_reads, const uint8_t *seq, con
 	const int grid = ctx->num_sms * per_sm;
 	if (big && (!sc.gtally || (uint64_t)grid * (kQueryThreads / 32) > sc.gtally_warps))
 		return mibf_fail(ctx, BBT_ERR_ARG, "the per-warp tally tables are missing or too small");
+	if (timed && (phase & kQueryBegin)) {
+		unsigned long long id = 0; /* unlike its address, never another stream's */
+		MIBF_TRY(ctx, cudaStreamGetId(s, &id));
+		if (id != ctx->scratch_stream)
+			MIBF_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_free, 0));
+		ctx->scratch_stream = id;
+	}
 	if (phase & kQueryBegin) {
 		MIBF_TRY(ctx, cudaMemsetAsync(batch_counts, 0, nc * 8, s));
 		MIBF_TRY(ctx, cudaMemsetAsync(sc.flags, 0, 4, s));
@@ -2086,6 +2096,8 @@ static int run_query_sc(bbt_mibf *ctx, uint64_t n_reads, const uint8_t *seq, con
 		mibf_commit_kernel<<<1, 256, 0, s>>>(batch_counts, ctx->d_counts, (uint32_t)nc, sc.flags,
 				total_reads);
 		MIBF_TRY(ctx, cudaGetLastError());
+		if (timed)
+			MIBF_TRY(ctx, cudaEventRecord(ctx->ev_free, s));
 	}
 	return BBT_OK;
 }

@@ -123,6 +123,10 @@ struct bbt_mibf {
 	cudaEvent_t c_copied[2] = {nullptr, nullptr}, c_computed[2] = {nullptr, nullptr};
 	uint64_t reads_seen = 0;
 	cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+	/* the end of the last query on the context's own scratch, which a query on another
+	 * stream waits for, and that stream's ID */
+	cudaEvent_t ev_free = nullptr;
+	unsigned long long scratch_stream = 0;
 	double last_kernel_ms = 0;
 	/* bucketed query (dense layout, mibf.cu): settings, then the scratch of
 	 * one call (frame offsets, offset samples, packed bases, frame validity

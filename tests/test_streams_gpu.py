@@ -70,3 +70,35 @@ def test_a_stream_that_the_caller_captures(tmp_path):
             assert np.array_equal(hits.cpu().numpy().view(np.uint64), want[0])
             assert np.array_equal(got.cpu().numpy().view(np.uint64), want[1])
         del graph
+
+
+@pytest.mark.parametrize("layout", [1, 2])
+def test_multi_index_queries_in_flight_together(tmp_path, layout):
+    import torch
+    from biobloom_b200.mibf import MIBFClassifier
+    from tests.test_mibf_gpu import _reads as mibf_reads
+    from tests.test_mibf_gpu import _targets
+    rng = np.random.default_rng(6)
+    targets = _targets(rng)
+    f = ol.MIBF.build(targets, list(range(1, len(targets) + 1)), k=25, h=3, occupancy=0.5)
+    f.store(str(tmp_path / "x"))
+    with open(tmp_path / "x_ids.txt", "w") as fh:
+        for i in range(len(targets)):
+            fh.write(f"{i + 1}\tt{i}\n")
+    c = MIBFClassifier(str(tmp_path / "x.bf"), layout=layout)
+    batches = [mibf_reads(rng, targets, n)[0] for n in (30000, 700)]
+    dev = [_device(b) for b in batches]
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    torch.cuda.synchronize()
+    with torch.cuda.stream(streams[0]):
+        want = [c.classify_device(*d, max_hits=4) for d in dev]
+    torch.cuda.synchronize()
+    got = []
+    for i in range(12):
+        with torch.cuda.stream(streams[i % 3]):
+            got.append((i % 2, c.classify_device(*dev[i % 2], max_hits=4)))
+    torch.cuda.synchronize()
+    for which, result in got:
+        for t, w in zip(result, want[which]):
+            assert torch.equal(t, w)
+    c.close()
