@@ -24,6 +24,13 @@ STEPS_DECISION, STEPS_FULL, STEPS_WIDE, STEPS_WIDE_FULL = 0, 1, 2, 3
 MODE_STD, MODE_ORDERED, MODE_BESTHIT, MODE_SCORES = 0, 1, 2, 3
 
 
+def stream_handle(stream):
+    """A torch stream as the library takes it.  The handle of torch's default stream is 0,
+    which in the library means the context's own stream: the default stream has another
+    name, cudaStreamLegacy."""
+    return ctypes.c_void_p(stream.cuda_stream or 1)
+
+
 class LibraryMissing(RuntimeError):
     pass
 

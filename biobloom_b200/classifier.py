@@ -282,10 +282,10 @@ class BioBloomClassifier:
             L.check(L.lib().bbt_classify_batch_scores(
                 self._ctx, ctypes.byref(b), ctypes.byref(r), ctypes.c_void_p(scores.data_ptr()),
                 ctypes.c_void_p(scores2.data_ptr()) if scores2 is not None else None,
-                ctypes.c_void_p(s.cuda_stream)), self._ctx)
+                L.stream_handle(s)), self._ctx)
             return hits, hits2, category
         L.check(L.lib().bbt_classify_batch(self._ctx, ctypes.byref(b), ctypes.byref(r),
-                                           ctypes.c_void_p(s.cuda_stream)), self._ctx)
+                                           L.stream_handle(s)), self._ctx)
         return hits, hits2, category
 
     def last_stats(self):
@@ -362,7 +362,7 @@ class ClassifyGraph:
         return n.value
 
     def launch(self, stream=None):
-        s = ctypes.c_void_p(stream.cuda_stream) if stream is not None else None
+        s = L.stream_handle(stream) if stream is not None else None
         L.check(L.lib().bbt_graph_launch(self._g, s), self._bbc._ctx)
 
     def close(self):

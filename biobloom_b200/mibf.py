@@ -149,7 +149,7 @@ class MIBFClassifier:
             hits.data_ptr(), max_hits, nh.data_ptr(), sat.data_ptr(), L.DEVICE)
         s = stream if stream is not None else torch.cuda.current_stream(dev)
         L.check_mibf(L.lib().bbt_mibf_classify_batch(self._ctx, ctypes.byref(b), ctypes.byref(r),
-                                                     ctypes.c_void_p(s.cuda_stream)), self._ctx)
+                                                     L.stream_handle(s)), self._ctx)
         return hits[:n], nh[:n], sat[:n]
 
     def sync(self):
