@@ -1658,7 +1658,8 @@ int bbt::mibf_reserve_rows(bbt_mibf *ctx, uint32_t rows)
 	return BBT_OK;
 }
 
-static std::vector<uint32_t> host_frame_counts(const bbt_batch *b, unsigned k);
+static std::vector<uint32_t> host_frame_counts(const bbt_batch *b, unsigned k,
+		uint64_t *most = nullptr);
 
 int bbt::mibf_rows_for(bbt_mibf *ctx, const uint64_t *off, const uint64_t *off2, uint64_t n)
 {
@@ -1675,14 +1676,19 @@ int bbt::mibf_rows_for(bbt_mibf *ctx, const uint64_t *off, const uint64_t *off2,
 	return ensure_min_count(ctx, fcs, ctx->stream);
 }
 
-static std::vector<uint32_t> host_frame_counts(const bbt_batch *b, unsigned k)
+/* The frame counts that occur in a batch (host offsets), and the frames of the read
+ * (pair) that has the most. */
+static std::vector<uint32_t> host_frame_counts(const bbt_batch *b, unsigned k, uint64_t *most)
 {
 	std::vector<uint32_t> fcs;
 	std::vector<uint8_t> seen;
+	uint64_t all = 0;
 	for (uint64_t r = 0; r < b->n_reads; ++r) {
 		const uint64_t l1 = b->offsets[r + 1] - b->offsets[r];
 		const uint64_t l2 = b->seq2 ? b->offsets2[r + 1] - b->offsets2[r] : 0;
-		const uint64_t fc = l1 >= k ? l1 - k + 1 : (l2 >= k ? l2 - k + 1 : 0);
+		const uint64_t f1 = l1 >= k ? l1 - k + 1 : 0, f2 = l2 >= k ? l2 - k + 1 : 0;
+		const uint64_t fc = f1 ? f1 : f2;
+		all = std::max(all, f1 + f2);
 		if (fc >= seen.size())
 			seen.resize(fc + 1, 0);
 		if (!seen[fc]) {
@@ -1690,6 +1696,8 @@ static std::vector<uint32_t> host_frame_counts(const bbt_batch *b, unsigned k)
 			fcs.push_back((uint32_t)fc);
 		}
 	}
+	if (most)
+		*most = all;
 	std::sort(fcs.begin(), fcs.end());
 	return fcs;
 }
@@ -2386,11 +2394,11 @@ extern "C" int bbt_mibf_classify_batch(bbt_mibf *ctx, const bbt_batch *b, bbt_mi
 				b->offsets2, res->hits, res->max_hits, res->n_hits, res->sat_count, s, most);
 	}
 	/* host batch: chunks through two slots, copies overlapping the launches */
-	rc = ensure_min_count(ctx, host_frame_counts(b, ctx->hd.k), s);
+	uint64_t most = 0;
+	rc = ensure_min_count(ctx, host_frame_counts(b, ctx->hd.k, &most), s);
 	if (rc)
 		return rc;
-	return classify_host_chunks(ctx, b, res, s,
-			mibf_most_frames(ctx, b->offsets, b->seq2 ? b->offsets2 : nullptr, b->n_reads));
+	return classify_host_chunks(ctx, b, res, s, most);
 }
 
 extern "C" int bbt_mibf_sync(bbt_mibf *ctx)
