@@ -21,11 +21,14 @@
  * over all k-mers (first numbers, new k-mers) with the slice's bits packed
  * between them.  Sequences that fit one chunk are copied to the device once.
  *
- * 20 Mbp (a 13.7 MB filter): 24 -> 15 ms, of which the kernels 3.1 -> 2.8.  The
- * first-number pass is the larger part of these (2.2 ms: 60 M atomics over 440
- * MB, 27 G/s, what isolated read-modify-writes of HBM reach); an insertion pass
- * of its own (0.35 ms), a copy of the sequences per pass and the redundancy
- * integral on one thread are gone.
+ * Whole calls, median of 25 passes and their range on one host (files and pageable
+ * copies included): 1 Mbp 32.0 (31.6 to 39.5) -> 9.5 ms (7.8 to 13.0), 5 Mbp 8.0 (7.8 to
+ * 8.2) -> 6.5 (6.2 to 9.4), 20 Mbp (a 13.7 MB filter) 20.5 (20.2 to 21.3) -> 19.9 (18.9 to
+ * 25.1): most of the last is host work, its kernels take 3.1 -> 2.8 ms.  The first-number
+ * pass is the larger part of these (2.2 ms: 60 M atomics over 440 MB, 27 G/s, what
+ * isolated read-modify-writes of HBM reach); an insertion pass of its own (0.35 ms), a copy
+ * of the sequences per pass and the redundancy integral on one thread (up to 2^20 terms)
+ * are gone.
  */
 #include <cuda_runtime.h>
 
@@ -186,6 +189,9 @@ extern "C" int bbt_make_filter(const char *seq, const uint64_t *offsets, uint64_
 	cudaError_t e = cudaSetDevice(device);
 	if (e != cudaSuccess)
 		return cuda_fail(nullptr, e, "cudaSetDevice");
+	int sms = 0;
+	if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess)
+		return cuda_fail(nullptr, e, "cudaDeviceGetAttribute");
 	uint32_t *d_words = nullptr;
 	uint8_t *d_seq = nullptr;
 	unsigned long long *d_counts = nullptr;
@@ -272,7 +278,7 @@ extern "C" int bbt_make_filter(const char *seq, const uint64_t *offsets, uint64_
 			idx0 += frames;
 		}
 		if (firsts) {
-			const unsigned grid = (unsigned)std::min<uint64_t>((sp + 255) / 256, 148 * 16);
+			const unsigned grid = (unsigned)std::min<uint64_t>((sp + 255) / 256, 16ull * sms);
 			if (narrow)
 				pack_bits_kernel<<<grid, 256>>>((const uint32_t *)d_first, lo, sp, d_words);
 			else
