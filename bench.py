@@ -574,7 +574,7 @@ def run_gpu(args):
     achieved = alg_bytes / (k_persistent * 1e-3) / 1e9
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": peak_kind,
-                "kernel": "classify path (scan + hash pass + filter pass)",
+                "kernel": "lane_kernel (a launch per filter)",
                 "classify_ms": k_persistent, "algorithmic_bytes_per_launch": alg_bytes}
     if best == L.PATH_FILTER_MAJOR:
         # each 68.5 MB filter is probed out of L2: the ceiling is the random
@@ -593,7 +593,7 @@ def run_gpu(args):
                          "hbm_peak_kind": peak_kind})
     tpr = traffic_per_read()
     roofline.update({"traffic": (tpr * n_reads if tpr else None),
-                     "traffic_note": "filter pass DRAM read+write per read from the committed "
+                     "traffic_note": "lane kernel DRAM read+write per read from the committed "
                                      "ncu capture, scaled to the step's reads"})
     value = world * n_reads / (ms_persistent * 1e-3)
     line = {
@@ -1059,6 +1059,13 @@ def run_single(args):
         bbc.set_launch(path=L.PATH_PERSISTENT)
     bbc.classify_device(d1, doff, hits=hits, category=cat, stream=stream)  # warm-up, same sizes
     stream.synchronize()
+    launch = min(tune["reads_per_launch"] or n, n)
+    if launch < n:
+        bbc.classify_device(d1, doff[:launch + 1], stream=stream)
+    kernels_per_launch = bbc.last_stats()["kernels"]
+    # the kernel that takes launches of so many reads (lane_rule, csrc/lane.cu)
+    by_lane = (tune["path"] in (L.PATH_PERSISTENT, L.PATH_FILTER_MAJOR) and
+               tune["steps"] == L.STEPS_DECISION and launch >= 160_000)
     hits.zero_()
     graph = None
     if tune["path"] == L.PATH_BUCKETED:
@@ -1076,7 +1083,6 @@ def run_single(args):
     clk = clocks.stop()
     batched_ok = bool(torch.equal(hits, want_hits))
     if graph is not None:
-        kernels_per_launch = 3 if (tune["long_bases"] and tune["path"] != L.PATH_PLAIN) else 2
         batched_launches = graph.launches * kernels_per_launch
     else:
         batched_step()
@@ -1182,7 +1188,8 @@ def run_single(args):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_kind": peak_kind, "traffic": None,
                 "kernel": {L.PATH_BUCKETED: "bucketed path (sweeps, resolve, walk)"}.get(
-                    tune["path"], "classify_kernel (tuned configuration)"),
+                    tune["path"], "lane_kernel" if by_lane else
+                    "classify_kernel (tuned configuration)"),
                 "classify_ms": k_ms, "algorithmic_bytes_per_launch": alg_bytes}
     if l2_resident:
         # the filter is probed out of L2: the ceiling is the random 4-byte
@@ -1206,9 +1213,9 @@ def run_single(args):
                                            ctypes.byref(rate)))
         issued_rate = issued / (k_ms * 1e-3)
         tpr = traffic_per_read("classify_varlen_dram.json")
-        if tpr and tune["path"] != L.PATH_BUCKETED:
+        if tpr and by_lane:
             roofline["traffic"] = tpr * n
-            roofline["traffic_note"] = ("persistent kernel DRAM read+write per read from the "
+            roofline["traffic_note"] = ("lane kernel DRAM read+write per read from the "
                                         "committed ncu capture of 400k reads of this workload, "
                                         "scaled to the step's reads")
         roofline["random_gather"] = {
@@ -1835,7 +1842,9 @@ def run_mibf(args):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": (tpr * n if tpr else None),
-                     "kernel": "mibf_query_kernel", "kernel_ms": kernel_ms,
+                     "kernel": ("mibf_scan_kernel" if dense and args.targets < 1024 and
+                                args.mibf_bucketing <= 0 else "mibf_query_kernel"),
+                     "kernel_ms": kernel_ms,
                      "algorithmic_bytes_per_launch": alg_bytes,
                      "algorithmic_bytes_note": ("32 B sector per probe (dense ID map)" if dense else
                                                 "32 B block sector per probe + 32 B ID sector "

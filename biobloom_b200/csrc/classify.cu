@@ -320,8 +320,8 @@ __global__ void summarize_kernel(uint64_t *__restrict__ h1, uint64_t *__restrict
 		uint64_t n, uint32_t nf, uint32_t words, int inclusive, int ordered, uint32_t *category,
 		unsigned long long *counts)
 {
-	/* 32-bit counters: a block counts at most the batch's reads of one grid
-	 * stride, and a shared-memory increment of a 32-bit word is one instruction
+	/* 32-bit counters: a block counts its share of the batch's reads, n over the
+	 * number of blocks, and a shared-memory increment of a 32-bit word is one instruction
 	 * for all lanes of a warp that hit the same counter, where a 64-bit one is a
 	 * compare-and-swap loop that serialises them */
 	extern __shared__ uint32_t sc[];

@@ -53,12 +53,12 @@ extern "C" {
 /* ---- kernel paths ---- */
 #define BBT_PATH_AUTO 0        /* persistent work-stealing path, tuned */
 #define BBT_PATH_PLAIN 1       /* one warp per read, one launch per batch */
-#define BBT_PATH_PERSISTENT 2  /* persistent work-stealing kernels: a read per lane from
-                                  20,000 reads on (28,000 over filters in HBM, up to 60,000
-                                  over many filters that fit L2 together), a read per warp
-                                  below */
-#define BBT_PATH_FILTER_MAJOR 3 /* one filter after another: a read per lane as above, below
-                                  that hashes stored once and (filter, read) items */
+#define BBT_PATH_PERSISTENT 2  /* persistent work-stealing kernels: a read per lane or a read
+                                  per warp, by the number of reads (from 20,000 to 160,000 on,
+                                  by the filters' sizes) and, below where the first always
+                                  pays, by their lengths */
+#define BBT_PATH_FILTER_MAJOR 3 /* one filter after another: a read per lane as above, or
+                                  hashes stored once and (filter, read) items */
 #define BBT_PATH_BUCKETED 4    /* probes sorted by filter address (filters far above L2) */
 
 typedef struct bbt_ctx bbt_ctx;
@@ -318,15 +318,17 @@ int bbt_classify_batch_scores(bbt_ctx *ctx, const bbt_batch *batch, bbt_result *
 		double *scores, double *scores2, void *stream);
 
 /* Kernel path and launch shape (BBT_PATH_*, warps per block 4 or 8, frames
- * per lane when hashing 4 or 8); 0 keeps the current value.  Used by the
- * tuner; no reference counterpart (the reference's only knob is -t threads,
- * BioBloomCategorizer.cpp:243-249). */
+ * per lane when hashing 4 or 8); 0 keeps the current value.  The shape is that of
+ * the kernels with a read per warp; the one with a read per lane has its own.
+ * Used by the tuner; no reference counterpart (the reference's only knob is -t
+ * threads, BioBloomCategorizer.cpp:243-249). */
 int bbt_set_launch(bbt_ctx *ctx, int path, int warps_per_block, int frames_per_lane);
 
-/* Read order of the persistent kernel: reads of at least long_bases bases are
- * started first (longest-processing-first scheduling, so that a long read does
- * not start last and hold the end of the launch); 0 = index order.  Results do
- * not depend on it.  No reference counterpart. */
+/* Read order of the persistent kernel with a read per warp: reads of at least
+ * long_bases bases are started first (longest-processing-first scheduling, so that a
+ * long read does not start last and hold the end of the launch); 0 = index order.
+ * The kernel with a read per lane always starts with the long ones.  Results do not
+ * depend on it.  No reference counterpart. */
 int bbt_set_schedule(bbt_ctx *ctx, uint64_t long_bases);
 
 /* Settings of the bucketed path (BBT_PATH_BUCKETED): each round's requests
@@ -349,7 +351,10 @@ int bbt_set_bucketing(bbt_ctx *ctx, unsigned bucket_shift, unsigned phase_split,
  * filters fit in L2; 4 or 8 warps per block; 4 or 8 frames per lane; the
  * persistent path with either step size of bbt_set_steps), keep
  * the fastest, then pick the reads per launch (64k, 256k, 1M or the whole
- * sample) for it, and leave the context set to the result.  The summary
+ * sample) for it, and leave the context set to the result.  Tune on a sample of the
+ * size of the batches to come: a smaller one compares the kernels that take batches
+ * of its size, and steps other than BBT_STEPS_DECISION, once chosen, keep later
+ * batches of any size on the kernel with a read per warp.  The summary
  * counters are left as they were.  No reference counterpart (the reference's
  * only knob is -t).
  */
@@ -364,15 +369,16 @@ typedef struct {
 } bbt_tune;
 int bbt_autotune(bbt_ctx *ctx, const bbt_batch *sample, bbt_tune *out);
 
-/* Steps of the persistent path's warp kernel (the one with a read per lane takes
- * the batches above where this is BBT_STEPS_DECISION).  Each step of a warp probes up to 32 frames
- * of a read, one per lane, or up to 64 with two frames per lane (WIDE: twice
- * the filter reads in flight, for filters in HBM where the kernel waits on
+/* Steps of the persistent path's kernel with a read per warp.  Each step of a warp
+ * probes up to 32 frames of a read, one per lane, or up to 64 with two frames per lane
+ * (WIDE: twice the filter reads in flight, for filters in HBM where the kernel waits on
  * them).  With SIMPLE and BINOMIAL scoring, DECISION steps are sized to the
  * frames that could still decide the read (fewer probes: filters in HBM) and
  * FULL steps are always full (fewer steps and instructions: filters held in
- * L2).  BBT_STEPS_DECISION is the default; bbt_autotune tries all four.
- * Results do not depend on it.  No reference counterpart. */
+ * L2).  BBT_STEPS_DECISION is the default, and the one with which the kernel with a
+ * read per lane takes the batches that it is faster for (1M reads over a filter in L2:
+ * 0.62 ms, 2.7 by warps); the others keep all batches on warps.  bbt_autotune tries all
+ * four.  Results do not depend on it.  No reference counterpart. */
 #define BBT_STEPS_DECISION 0
 #define BBT_STEPS_FULL 1
 #define BBT_STEPS_WIDE 2
