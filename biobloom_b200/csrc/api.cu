@@ -224,7 +224,7 @@ extern "C" int bbt_close(bbt_ctx *ctx)
 	}
 	if (ctx->ev_start)
 		cudaEventDestroy(ctx->ev_start);
-	for (cudaEvent_t e : ctx->ev_stop)
+	for (cudaEvent_t e : {ctx->ev_stop[0], ctx->ev_stop[1], ctx->ev_legacy})
 		if (e)
 			cudaEventDestroy(e);
 	if (ctx->ev_k0)
@@ -478,6 +478,7 @@ extern "C" int bbt_open(const char *const *bf_paths, int n_filters, const bbt_pa
 	OPEN_TRY(cudaEventCreate(&ctx->ev_start));
 	for (cudaEvent_t &e : ctx->ev_stop)
 		OPEN_TRY(cudaEventCreate(&e));
+	OPEN_TRY(cudaEventCreateWithFlags(&ctx->ev_legacy, cudaEventDisableTiming));
 	OPEN_TRY(cudaEventCreate(&ctx->ev_k0));
 	OPEN_TRY(cudaEventCreate(&ctx->ev_k1));
 	for (Slot &s : ctx->slot) {
@@ -815,9 +816,11 @@ static cudaError_t mark_stop(bbt_ctx *ctx, cudaStream_t s)
 /* Two-pass filter-major classification of one batch (all filters share k):
  * scan of padded frame counts, a host read of the per-block totals to cut the
  * batch into sub-batches whose frames fit the scratch, then hash pass and
- * filter pass per sub-batch. */
-static int run_two_pass(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s,
-		const ScoreArgs *sa = nullptr, bool classify = true)
+ * filter pass per sub-batch.  With `ask`, whose counts are on their way to
+ * h_lane_stats, the wait also decides whether the lane kernel takes the batch
+ * instead (*lanes; nothing else is done). */
+static int run_two_pass(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s, const ScoreArgs *sa,
+		bool classify, const LaneRule *ask, bool *lanes)
 {
 	const uint64_t total = a.n * a.mates;
 	const uint64_t B = two_pass_block_reads();
@@ -842,6 +845,11 @@ static int run_two_pass(bbt_ctx *ctx, ClassifyArgs &a, cudaStream_t s,
 	CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_tp_sums, ctx->d_tp_sums,
 			(nb + 1) * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
 	CUDA_TRY(ctx, cudaStreamSynchronize(s));
+	if (ask && lane_takes(*ask, ctx->h_lane_stats, total)) {
+		ctx->last.kernels += 2; /* scans */
+		*lanes = true;
+		return BBT_OK;
+	}
 	const unsigned long long *sums = ctx->h_tp_sums;
 	/* frame slots per sub-batch (8 bytes of hash each) */
 	const uint64_t budget = ctx->p.max_batch_bases ? std::max<uint64_t>(ctx->p.max_batch_bases, 32)
@@ -1278,8 +1286,14 @@ static LaneUse lane_use(const bbt_ctx *ctx, const LaunchConfig &lc, uint64_t tot
 	if (lc.path != BBT_PATH_FILTER_MAJOR &&
 			!(lc.path == BBT_PATH_PERSISTENT && lc.steps == BBT_STEPS_DECISION))
 		return kLaneNo;
-	rule = lane_rule(ctx->hf.data(), ctx->nf, ctx->mode == BBT_MODE_BESTHIT ||
-			ctx->mode == BBT_MODE_SCORES, total);
+	LaneAim aim;
+	aim.scores = ctx->mode == BBT_MODE_BESTHIT || ctx->mode == BBT_MODE_SCORES;
+	aim.harmonic = ctx->p.scoring == BBT_SCORE_HARMONIC;
+	aim.length = ctx->p.scoring == BBT_SCORE_LENGTH;
+	aim.quick = aim.length || (!aim.scores && ctx->p.scoring != BBT_SCORE_BINOMIAL &&
+			ctx->p.score > 0.3);
+	aim.host = lc.path == BBT_PATH_FILTER_MAJOR && ctx->same_k;
+	rule = lane_rule(ctx->hf.data(), ctx->nf, aim, total);
 	if (total < rule.least ||
 			!lane_supports(ctx->hf.data(), ctx->nf, ctx->p.streak_threshold, total))
 		return kLaneNo;
@@ -1422,11 +1436,8 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 		CUDA_TRY(ctx, launch_lane_list(a, ls, ctx->num_sms, s));
 		ctx->last.kernels += 1;
 		if (lane == kLaneAsk && two_pass) {
-			/* these passes are planned on the host, with a short wait: so is the choice */
 			CUDA_TRY(ctx, cudaMemcpyAsync(ctx->h_lane_stats, ls.ctr, kLaneStats *
 					sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-			CUDA_TRY(ctx, cudaStreamSynchronize(s));
-			lane = lane_takes(rule, ctx->h_lane_stats, a.n * a.mates) ? kLaneYes : kLaneNo;
 		} else if (lane == kLaneAsk) {
 			a.lane_stats = ls.ctr;
 			a.lane_rule = rule;
@@ -1440,13 +1451,16 @@ static int run_kernels(bbt_ctx *ctx, ClassifyArgs &a, uint32_t *d_cat, cudaStrea
 	}
 	const bool stored = best || want_scores; /* scores go to memory (lane, two-pass) */
 	int rc = BBT_OK;
-	if (lane) {
-		rc = run_lane(ctx, a, s, stored ? &ps : nullptr, !best);
-	} else if (two_pass) {
+	if (two_pass && lane != kLaneYes) {
+		bool lanes = false;
 		rc = best ? BBT_OK : zero_hits(ctx, a, s);
 		if (!rc)
-			rc = run_two_pass(ctx, a, s, stored ? &ps : nullptr, !best);
+			rc = run_two_pass(ctx, a, s, stored ? &ps : nullptr, !best,
+					lane == kLaneAsk ? &rule : nullptr, &lanes);
+		lane = lanes ? kLaneYes : kLaneNo;
 	}
+	if (!rc && lane)
+		rc = run_lane(ctx, a, s, stored ? &ps : nullptr, !best);
 	if (!rc && best && (lane || two_pass)) {
 		CUDA_TRY(ctx, launch_best_hits(a, ps.scores, ctx->num_sms, s));
 		ctx->last.kernels += 1;
@@ -1556,13 +1570,28 @@ static int classify_device_batch(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r
 static int classify_device(bbt_ctx *ctx, const bbt_batch *b, bbt_result *r, cudaStream_t s,
 		double *const *scores = nullptr)
 {
+	/* the default stream: between two events on the context's own, where launches cost the
+	 * host less (4,000 reads over ten filters in L2, filter-major: 150 us, 167 there) */
+	const bool legacy = s == cudaStreamLegacy;
+	if (legacy) {
+		CUDA_TRY(ctx, cudaEventRecord(ctx->ev_legacy, cudaStreamLegacy));
+		s = ctx->stream;
+		CUDA_TRY(ctx, cudaStreamWaitEvent(s, ctx->ev_legacy, 0));
+	}
 	cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
 	CUDA_TRY(ctx, cudaStreamIsCapturing(s, &st));
 	ctx->callers_capture = !ctx->capturing && st != cudaStreamCaptureStatusNone;
-	const int rc = classify_device_batch(ctx, b, r, s, scores);
+	int rc = classify_device_batch(ctx, b, r, s, scores);
 	ctx->callers_capture = false;
 	if (ctx->claimed) /* it failed on the way: what it launched still uses the scratch */
 		mark_stop(ctx, s);
+	if (legacy) {
+		cudaError_t e = cudaEventRecord(ctx->ev_legacy, s);
+		if (e == cudaSuccess)
+			e = cudaStreamWaitEvent(cudaStreamLegacy, ctx->ev_legacy, 0);
+		if (!rc && e != cudaSuccess)
+			rc = cuda_fail(ctx, e, "cudaStreamWaitEvent(default stream)");
+	}
 	return rc;
 }
 

@@ -199,7 +199,8 @@ __device__ void classify_read(const ClassifyArgs &a, uint64_t r, uint32_t f0, ui
 /* A read above kWindowBases against all filters in windows of up to 256 frames
  * (lane_long_item): a batch's longest read sets the time of a small batch, and a
  * step of 32 frames costs the latency of h dependent probes just the same (4,000
- * reads of 50 bp to 10 kb over a 2.1 GB filter: 982 -> 295 us).  wmem: a warp's
+ * reads of 50 bp to 10 kb over a 2.1 GB filter: 982 -> 295 us).  Not for LENGTH, whose
+ * windows are 64 frames hashed as 256 (797 us against 629).  wmem: a warp's
  * hash window, which holds more than the tables and 16 words. */
 template <bool COUNT, int MODE>
 __device__ __noinline__ void classify_long(const ClassifyArgs &a, uint64_t r, unsigned char *wmem,
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(256, BBT_CLASSIFY_MIN_BLOCKS) classify_kernel(
 			uint64_t myword = 0;
 			const uint32_t mate = r >= a.n ? 1u : 0u;
 			const uint64_t i = r - (mate ? a.n : 0);
-			if (!WIDE && a.long_bases && a.off[mate][i + 1] - a.off[mate][i] > a.long_bases) {
+			if (!WIDE && MODE != BBT_SCORE_LENGTH && a.long_bases && a.off[mate][i + 1] - a.off[mate][i] > a.long_bases) {
 				unsigned long long acc[3] = {0, 0, 0};
 				classify_long<COUNT, MODE>(a, r, smem + warp * window_stride<SEG>(a.kmax), lane,
 						myword, COUNT ? acc : nullptr);

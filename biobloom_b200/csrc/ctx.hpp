@@ -177,6 +177,7 @@ struct bbt_ctx {
 	 * other streams wait for before they use it; [0]: of the last call that did not */
 	cudaEvent_t ev_start = nullptr, ev_stop[2] = {nullptr, nullptr};
 	int last_stop = 0;                     /* of the last call */
+	cudaEvent_t ev_legacy = nullptr;       /* between the default stream and the context's */
 	bool claimed = false;                  /* this call uses the scratch */
 	unsigned long long scratch_stream = 0; /* ID of the stream that used it last */
 	cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr; /* around the last classify kernel */

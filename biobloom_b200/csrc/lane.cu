@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) lane_list_kernel(ClassifyArgs a, uint32_t
 		unsigned long long *stats)
 {
 	__shared__ uint64_t sums[8];
-	__shared__ uint32_t tops[8];
+	__shared__ uint32_t tops[8], at[2][8], first[2];
 	const uint64_t total = a.n * a.mates;
 	const int lane = threadIdx.x & 31;
 	const unsigned below = (1u << lane) - 1u;
@@ -117,23 +117,32 @@ __global__ void __launch_bounds__(256) lane_list_kernel(ClassifyArgs a, uint32_t
 			bases += (uint32_t)len;
 			longest = max(longest, (uint32_t)len);
 		}
+		if (!__syncthreads_or(len > kLaneShortBases))
+			continue;
+		/* places in the list: one atomic addition of the block for each kind */
 		const unsigned lm = __ballot_sync(kFull, len > kLaneMaxBases);
 		const unsigned mm = __ballot_sync(kFull, len > kLaneShortBases) & ~lm;
-		if (!(lm | mm))
-			continue;
-		unsigned long long lb = 0, mb = 0;
 		if (lane == 0) {
-			if (lm)
-				lb = atomicAdd(stats + kLaneLong, (unsigned long long)__popc(lm));
-			if (mm)
-				mb = atomicAdd(stats + kLaneMid, (unsigned long long)__popc(mm));
+			at[0][threadIdx.x >> 5] = __popc(lm);
+			at[1][threadIdx.x >> 5] = __popc(mm);
 		}
-		lb = __shfl_sync(kFull, lb, 0);
-		mb = __shfl_sync(kFull, mb, 0);
+		__syncthreads();
+		if (threadIdx.x < 2) {
+			uint32_t n = 0;
+			for (int i = 0; i < 8; ++i) {
+				const uint32_t c = at[threadIdx.x][i];
+				at[threadIdx.x][i] = n;
+				n += c;
+			}
+			first[threadIdx.x] = n ? (uint32_t)atomicAdd(stats + (threadIdx.x ? kLaneMid : kLaneLong),
+					(unsigned long long)n) : 0u;
+		}
+		__syncthreads();
 		if ((lm >> lane) & 1u)
-			list[lb + __popc(lm & below)] = (uint32_t)r;
+			list[first[0] + at[0][threadIdx.x >> 5] + __popc(lm & below)] = (uint32_t)r;
 		else if ((mm >> lane) & 1u)
-			list[total - 1 - (mb + __popc(mm & below))] = (uint32_t)r;
+			list[total - 1 - (first[1] + at[1][threadIdx.x >> 5] + __popc(mm & below))] = (uint32_t)r;
+		__syncthreads(); /* read before the next ones are written */
 	}
 	const uint64_t sum = __reduce_add_sync(kFull, bases & 0xFFFFu) +
 			((uint64_t)__reduce_add_sync(kFull, bases >> 16) << 16);
@@ -275,11 +284,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 	LaneWarp<MODE> &w = warps[warp];
 	unsigned long long acc[3] = {0, 0, 0}; /* words read, frames hashed, words of the
 	                                          sequential algorithm */
-	if (warp == 0)
-		lane_tables<PACKED>(tab, g.F.k, lane);
-	if (MODE == SCORE_HARMONIC && threadIdx.x < kHarmTerms)
-		terms[threadIdx.x] = harmonic_term(threadIdx.x);
-	if (threadIdx.x == 32) {
+	if (threadIdx.x == 0) {
 		const unsigned long long nmid = g.stats[kLaneMid];
 		const bool mids = lane_mids<SCORE>(g.F.keep != 0, nmid, a.n * a.mates);
 		sh.nlong = (uint32_t)g.stats[kLaneLong];
@@ -294,6 +299,11 @@ __global__ void __launch_bounds__(kLaneWarps * 32, kLaneMinBlocks) lane_kernel(
 	__syncthreads();
 	if (!sh.go)
 		return;
+	if (warp == 0)
+		lane_tables<PACKED>(tab, g.F.k, lane);
+	if (MODE == SCORE_HARMONIC && threadIdx.x < kHarmTerms)
+		terms[threadIdx.x] = harmonic_term(threadIdx.x);
+	__syncthreads();
 
 	/* listed reads, a warp each */
 	if (sh.listed && (warp < (int)sh.warps || sh.help)) {
@@ -536,16 +546,23 @@ bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64
  * reads), the other kernels' time grows with the bases; ragged reads below are 50 to 300
  * bases, log-uniform.
  *
+ * Measured with SIMPLE scoring at 0.15, three hashes and k = 25 unless said otherwise.
+ *
  * - one filter in L2: from 20,000 reads on where these are short and of much the same
  *   length (20,000 / 28,000 / 40,000 reads, 3.4 MB: 150 bases 95 / 93 / 106 us against
  *   115 / 135 / 166, 300 bases 145 / 151 / 172 against 144 / 173 / 217, 600 bases 258 /
  *   260 / 300 against 206 / 254 / 327, ragged 154 / 153 / 171 against 119 / 139 / 176),
- *   from 40,000 on always; scores, every frame of which is walked, from 20,000 on always.
+ *   from 40,000 on always, with more than four hashes from 60,000 (six, 40,000 reads: 600
+ *   bases 448 against 397, ragged 218 against 200); scores, every frame of which is walked,
+ *   from 20,000, or 28,000 (20,000 ragged reads, six hashes: 232 against 183).  With LENGTH
+ *   scoring, whose windows are short, only without long reads (60,000 ragged reads with
+ *   them 890 against 771).
  * - two to four that fit L2 together: the filter-major passes hash a read once for all of
  *   them.  Four of 3.4 MB, 28,000 / 50,000 reads: 150 bases 270 / 326 us against 297 /
  *   466, 600 bases 914 / 1110 against 946 / 1608; 28,000 / 100,000 ragged ones 501 / 874
  *   against 334 / 805.  Scores of ragged reads 522 against 448 at 28,000, 571 against 577
- *   at 40,000.
+ *   at 40,000.  The filter-major path asks from 40,000 reads on, where the answer costs less
+ *   than it brings (28,000 of 150 bases 321 against 302).
  * - more that fit L2 together: likewise, and a launch's latency for each.  Ten of 3.4 MB
  *   meet at 50,000 reads (150 bases 751 against 872, 300 bases 1423 against 1634), thirty
  *   at 75,000 (80,000: 3007 against 3478); scores at 20,000 (150 bases 611 against 639) and
@@ -559,35 +576,56 @@ bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64
  * - one filter in HBM: a lane waits longer for its probes.  28,000 / 80,000 / 160,000 reads,
  *   2.1 GB: 100 bases 116 / 216 / 331 us against 144 / 281 / 508, 150 bases 154 / 305 / 487
  *   against 164 / 339 / 616, 300 bases 265 / 569 / 940 against 240 / 535 / 996; 40,000 /
- *   60,000 ragged ones 248 / 305 against 205 / 275.  Scores: 100 bases 185 / 437 / 653
+ *   60,000 ragged ones 248 / 305 against 205 / 275; threshold 0.8, 100,000 of 150 bases 567
+ *   against 518.  Scores: 100 bases 185 / 437 / 653
  *   against 210 / 456 / 841, 150 bases 266 / 691 / 1053 against 286 / 655 / 1211, 300 bases
  *   515 / 1437 / 2190 against 501 / 1234 / 2375.
  * - several, one or more of them in HBM: the read-major kernel's probes of all filters
  *   overlap.  3.4 MB and 2.1 GB, 28,000 / 40,000 ragged reads 334 / 383 us against 249 /
- *   315, scores of 50,000 / 160,000 reads of 150 bases 543 / 1310 against 490 / 1406. */
-LaneRule lane_rule(const FilterDev *hf, uint32_t nf, bool scores, uint64_t reads)
+ *   315, scores of 50,000 / 160,000 reads of 150 bases 543 / 1310 against 490 / 1406.
+ * - several filters and early decisions: the passes and the read-major kernel stop at
+ *   them for all filters at once.  Four of 3.4 MB, threshold 0.8: 28,000 reads of 300 bases
+ *   529 us against 388; LENGTH, 100,000 ragged reads with long ones 4740 against 2422, best
+ *   hits of 20,000 of 150 bases over ten 606 against 419.  HARMONIC scoring of long reads:
+ *   100,000 ragged ones, best hits over four 9364 against 6559. */
+LaneRule lane_rule(const FilterDev *hf, uint32_t nf, const LaneAim &aim, uint64_t reads)
 {
 	const uint64_t always = ~0ull;
 	const uint32_t none = ~0u, any = 0, free = ~0u;
+	const bool scores = aim.scores;
 	uint64_t bytes = 0, most = 0;
+	uint32_t h = 0;
 	for (uint32_t i = 0; i < nf; ++i) {
 		bytes += hf[i].m / 8;
 		most = std::max(most, hf[i].m / 8);
+		h = std::max(h, hf[i].h);
 	}
+	if (nf > 1 && aim.quick)
+		return {most > kLaneKeepBytes ? 160000u : 150000u, always, 64, none, free, true};
 	if (most > kLaneKeepBytes && nf > 1)
-		return {160000, always, 8, 8, free, false};
+		return {160000, always, 8, aim.harmonic ? none : 8, free, false};
 	if (most > kLaneKeepBytes)
-		return {28000, 160000, 8, any, scores ? 130u : 170u, reads < 100000};
+		return {28000, aim.length ? always : 160000, 8, any, 130, true};
+	if (nf == 1 && scores)
+		return {aim.length ? 28000u : 20000u, h > 4 || aim.length ? 28000u : 20000u, any, any, free,
+				true};
+	if (nf == 1) {
+		const uint32_t sure = h > 4 || aim.length ? 60000 : 40000;
+		const bool few = reads < sure;
+		return {20000, aim.length ? always : sure, few ? 8 : any, aim.length ? none : any,
+				reads < 28000 ? 170u : few ? 250u : free, few};
+	}
+	if (bytes > kLaneKeepBytes && aim.harmonic)
+		return {28000, always, 64, none, free, true};
 	if (bytes > kLaneKeepBytes)
 		return {28000, 60000, any, scores && reads < 40000 ? 64 : any, free, true};
-	if (nf == 1)
-		return {20000, scores ? 20000u : 40000u, 8, any, reads < 28000 ? 170u : 250u, true};
 	if (nf <= 4)
-		return {20000, scores ? 40000u : 150000u, reads < 40000 ? 8 : any, any,
+		return {aim.host ? 40000u : 20000u, aim.harmonic ? always : scores ? 40000u : 150000u,
+				aim.harmonic ? 64u : reads < 40000 ? 8u : any, aim.harmonic ? none : any,
 				reads < 28000 ? 120u : free, true};
 	if (scores)
-		return {nf <= 10 ? 20000 : std::max<uint64_t>(28000, 1400ull * nf), always, 64, none, free,
-				true};
+		return {nf <= 10 ? (aim.host ? 28000 : 20000) : std::max<uint64_t>(28000, 1400ull * nf),
+				always, 64, none, free, true};
 	return {std::max<uint64_t>(std::min<uint64_t>(60000, 5000ull * nf), 2500ull * nf), always, 64,
 			none, free, true};
 }

@@ -62,7 +62,13 @@ struct LaneScratch {
 /* Whether the lane kernel can take these filters and options at all, and which
  * batches it is the faster one for. */
 bool lane_supports(const FilterDev *hf, uint32_t nf, uint32_t streak_thr, uint64_t total_reads);
-LaneRule lane_rule(const FilterDev *hf, uint32_t nf, bool scores, uint64_t reads);
+struct LaneAim {
+	bool scores;   /* every frame is walked (BESTHIT, SCORES) */
+	bool quick;    /* decided after few frames: LENGTH, thresholds above 0.3 */
+	bool harmonic, length;
+	bool host;     /* the lengths are read on the host (filter-major path) */
+};
+LaneRule lane_rule(const FilterDev *hf, uint32_t nf, const LaneAim &aim, uint64_t reads);
 
 /* Counters of a launch (which is a kernel per filter, after one that lists the
  * longer reads). */

@@ -79,10 +79,14 @@ def test_one_small_filter(tmp_path, kind, n, paired, best):
     _check(tmp_path, np.random.default_rng(n + paired), [25], kind, n, paired, best)
 
 
-@pytest.mark.parametrize("scoring,score", [(ol.HARMONIC, 0.15), (ol.LENGTH, 40)])
-def test_other_scoring(tmp_path, scoring, score):
-    for kind in ("ragged", "mids"):
-        _check(tmp_path, np.random.default_rng(5), [25], kind, 41000, False, False, scoring, score)
+@pytest.mark.parametrize("ks,scoring,score,kind,n", [
+    ([25], ol.HARMONIC, 0.15, "ragged", 61000), ([25], ol.HARMONIC, 0.15, "mids", 61000),
+    ([25, 25], ol.HARMONIC, 0.15, "even", 28100), ([25], ol.LENGTH, 40, "even", 20100),
+    ([25], ol.LENGTH, 40, "even", 61000), ([25], ol.LENGTH, 40, "long", 20100),
+    ([25, 21], ol.LENGTH, 40, "even", 151000), ([25], ol.SIMPLE, 0.8, "even", 20100),
+    ([25, 25], ol.SIMPLE, 0.8, "even", 151000)])
+def test_other_scoring(tmp_path, ks, scoring, score, kind, n):
+    _check(tmp_path, np.random.default_rng(n), ks, kind, n, False, False, scoring, score)
 
 
 @pytest.mark.parametrize("kind,n,best", [
@@ -94,18 +98,24 @@ def test_a_filter_larger_than_l2(tmp_path, kind, n, best):
     _check(tmp_path, np.random.default_rng(n), [25], kind, n, False, best, fpr=1.7e-5, h=1)
 
 
-@pytest.mark.parametrize("nf,kind,n,best,lane", [
-    (3, "even", 20100, False, True), (3, "ragged", 20100, False, False),
-    (3, "long", 20100, False, True), (3, "mids", 30000, False, False),
-    (3, "ragged", 150100, False, True), (3, "ragged", 40100, True, True),
-    (6, "even", 30100, False, True), (6, "ragged", 30100, False, False),
-    (6, "long", 30100, False, False), (6, "even", 20100, True, True),
-    (6, "mids", 30100, True, False)])
-def test_the_filter_major_path_asks_on_the_host(tmp_path, nf, kind, n, best, lane):
+def test_listed_reads_by_match_length(tmp_path):
+    _check(tmp_path, np.random.default_rng(3), [25], "long", 28100, False, False, ol.LENGTH, 40,
+           fpr=1.7e-5, h=1)
+
+
+@pytest.mark.parametrize("nf,kind,n,best,asked,lane", [
+    (3, "even", 28100, False, False, False), (3, "even", 40100, False, True, True),
+    (3, "ragged", 40100, False, True, False), (3, "long", 40100, False, True, True),
+    (3, "mids", 41000, False, True, False), (3, "ragged", 150100, False, False, True),
+    (3, "ragged", 40100, True, False, True), (6, "even", 30100, False, True, True),
+    (6, "ragged", 30100, False, True, False), (6, "long", 30100, False, True, False),
+    (6, "even", 28100, True, True, True), (6, "mids", 30100, True, True, False)])
+def test_the_filter_major_path_asks_on_the_host(tmp_path, nf, kind, n, best, asked, lane):
     stats = _check(tmp_path, np.random.default_rng(nf * 1000 + n), [25] * nf, kind, n, False, best,
                    glen=4000)
-    # summary, list, and a kernel a filter or two scans, hash and filter pass; best hits
-    assert stats["kernels"] == 2 + (nf if lane else 4) + best
+    # summary, best hits; the list; two scans, and hash and filter pass or a kernel a filter
+    assert stats["kernels"] == 1 + best + (asked or lane) + (2 if asked or not lane else 0) + \
+        (nf if lane else 2)
 
 
 @pytest.mark.parametrize("kind", ["even", "ragged"])
